@@ -41,6 +41,7 @@ constexpr unsigned kStatusNeighborOverflow = 1u;
 constexpr unsigned kStatusNonFinite = 2u;
 constexpr unsigned kStatusFixedOverflow = 4u;
 constexpr unsigned kStatusCellClamp = 8u;
+constexpr unsigned kStatusStalled = 16u;  // a barrier of the whole-step kernel ran out
 
 // accumulator lanes (ReplicaState::acc)
 enum AccLane : int {

@@ -109,11 +109,13 @@ void Engine::set_tuning(int tpa, int fuse_post, int unroll, int no_l1) {
   if (tpa == 0) {
     tuning_fixed_ = false;
     tuned_ = false;
+    whole_steps_ = false;
     return;
   }
   if (tpa != 1 && tpa != 2 && tpa != 4) throw InvalidArgument("threads per particle must be 1, 2 or 4.");
   if (unroll != 4 && unroll != 8) throw InvalidArgument("batch depth must be 4 or 8.");
   clear_graphs();
+  whole_steps_ = false;
   launch_.lj_tpa = tpa;
   launch_.lj_unroll = unroll;
   launch_.lj_no_l1 = no_l1 ? 1 : 0;
@@ -129,6 +131,17 @@ void Engine::tuning(int* tpa, int* fuse_post, int* unroll, int* no_l1, int* auto
   *autotuned = (tuned_ && !tuning_fixed_) ? 1 : 0;
 }
 
+// Steps in one persistent kernel or kernel by kernel.  k_run saves the
+// launches and the conditional node (~20 us of a step) and pays with one wave
+// of blocks sized by the list build's registers, which costs throughput once
+// the pair forces fill the GPU.  Measured, us per step, kernel by kernel ->
+// k_run: 250 beads 28 -> 16, 4,096 24 -> 16, 20,011 34 -> 26; 100,003 48 -> 46;
+// 1,048,576 241 -> 331.
+bool Engine::use_whole_steps() const {
+  constexpr uint32_t kWholeStepSlots = 65536;
+  return use_graphs_ && v_.n_slots <= kWholeStepSlots && !(layout_fixed_ && v_.list_by_q != 0);
+}
+
 // Times the force stage of a step (pair forces, bonded terms, second
 // half-kick and kinetic total) under every schedule on the current list and
 // keeps the fastest.  The kicks of the trial launches are undone.  With
@@ -136,6 +149,21 @@ void Engine::tuning(int* tpa, int* fuse_post, int* unroll, int* no_l1, int* auto
 void Engine::autotune() {
   TraceRange trace("beads.autotune");
   if (!initialized_) eval();
+  if (use_whole_steps()) {
+    if (v_.list_by_q != 0) {
+      v_.list_by_q = 0;
+      launch_.v = v_;
+      relayout_list();
+    }
+    clear_graphs();
+    whole_steps_ = true;
+    launch_.lj_tpa = 4;
+    launch_.lj_unroll = 4;
+    launch_.lj_no_l1 = 1;
+    launch_.fuse_post = 1;
+    tuned_ = true;
+    return;
+  }
   constexpr int kWarm = 1, kReps = 4;
   const bool log = [] {
     const char* e = std::getenv("BEADS_TUNE_LOG");
@@ -671,6 +699,10 @@ void Engine::upload_static(uint32_t n, const beads_system_desc* systems,
   uint32_t* d_cell_replica = dalloc<uint32_t>(C);
   v.chain_launches = dalloc<unsigned long long>(1);
   v.ke_part = dalloc<long long>(2ull * n * kKeBuckets);  // zeroed; emptied by every finish
+  run_.ctl = dalloc<RunControl>(1);
+  run_.work_atoms = dalloc<uint32_t>(n + 1);
+  run_.chunk_sum = dalloc<uint32_t>(run_scan_chunks(C));
+  run_.ke_odd = dalloc<long long>(2ull * n * kKeBuckets);
   cuda_check(cudaMemsetAsync(v.chain_launches, 0, sizeof(unsigned long long), stream_), "memset");
   LjCoeff* d_lj = dalloc<LjCoeff>(h_lj.size());
 
@@ -748,6 +780,9 @@ void Engine::upload_static(uint32_t n, const beads_system_desc* systems,
   launch_.need_kinetic = any_thermostat ? 1 : 0;
   launch_.any_dense = any_dense_ ? 1 : 0;
   launch_.any_sparse = any_sparse_ ? 1 : 0;
+  run_.any_dense = launch_.any_dense;
+  run_.any_sparse = launch_.any_sparse;
+  run_.need_kinetic = launch_.need_kinetic;
   {
     // One wave of 128-thread blocks (16 per SM) for the chain's per-slot
     // kernels when they walk the block list.
@@ -791,6 +826,10 @@ void Engine::check_status() {
         << ". Increase max_neighbors before consuming this neighbor list.";
       if (rep_.size() > 1) m << " (replica " << r << ")";
       throw NeighborOverflow(m.str());
+    }
+    if (s & kStatusStalled) {
+      cudaMemsetAsync(run_.ctl, 0, sizeof(RunControl), stream_);
+      throw CudaError("the step kernel's blocks did not meet at a barrier.");
     }
     if (s & kStatusFixedOverflow) {
       throw OverflowError("energy, virial or kinetic energy of a particle is not finite or "
@@ -945,7 +984,10 @@ void Engine::launch_counts(uint32_t& per_step, uint32_t& per_chain) {
 }
 
 void Engine::launch_chunk(uint32_t steps, bool obs_last) {
-  if (use_graphs_) {
+  if (whole_steps_) {
+    if (steps > (obs_last ? 1u : 0u)) launch_run(launch_, run_, steps - (obs_last ? 1u : 0u), false);
+    if (obs_last) launch_run(launch_, run_, 1, true);
+  } else if (use_graphs_) {
     cuda_check(cudaGraphLaunch(graph_for(steps, obs_last), stream_), "graph launch");
   } else {
     for (uint32_t s = 0; s < steps; ++s) record_step(obs_last && s + 1 == steps);
@@ -985,7 +1027,7 @@ bool Engine::run(uint64_t steps, uint64_t obs_every, const std::function<bool()>
     // log2(kChunkMax) + 1 distinct captured graphs (instantiated once each).
     uint64_t pow2 = 1;
     while (pow2 * 2 <= chunk) pow2 *= 2;
-    if (pow2 != chunk) {
+    if (pow2 != chunk && !whole_steps_) {
       chunk = pow2;
       obs = false;
     }
@@ -1026,16 +1068,22 @@ bool Engine::run(uint64_t steps, uint64_t obs_every, const std::function<bool()>
 
 void Engine::minimize(uint32_t iterations, float dmax, float fref) {
   TraceRange trace("beads.minimize");
+  // The descent steps in k_run, on slot rows; a staged context goes back to
+  // its layout afterwards (its next evaluation builds the list again).
+  const int by_q = v_.list_by_q;
+  v_.list_by_q = 0;
+  launch_.v = v_;
   StepLaunch l = launch_;
   l.sd_dmax = dmax;
   l.sd_fref = fref;
+  constexpr uint32_t kDescentChunk = 64;
   launch_rebuild(l, true);
-  for (uint32_t it = 0; it < iterations; ++it) {
-    launch_forces(l, false, true);
-    launch_pre(l, kPreDescent);
-    launch_rebuild(l, false);
+  for (uint32_t it = 0; it < iterations; it += kDescentChunk) {
+    launch_descent(l, run_, std::min(kDescentChunk, iterations - it));
   }
   sync();
+  v_.list_by_q = by_q;
+  launch_.v = v_;
   // The descent is set-up work: reset counters so a following run starts
   // like a fresh one.
   check_status();
@@ -1295,6 +1343,10 @@ void Engine::set_list_staged(bool staged) {
   layout_fixed_ = true;
   if ((v_.list_by_q != 0) == want) return;
   clear_graphs();
+  if (want && whole_steps_) {  // k_run reads slot rows: tune for the staged layout
+    whole_steps_ = false;
+    tuned_ = false;
+  }
   v_.list_by_q = want ? 1 : 0;
   launch_.v = v_;
   if (initialized_) relayout_list();

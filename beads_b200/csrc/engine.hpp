@@ -134,6 +134,9 @@ class Engine {
   void set_tuning(int tpa, int fuse_post, int unroll, int no_l1);
   void tuning(int* tpa, int* fuse_post, int* unroll, int* no_l1, int* autotuned) const;
   void autotune();
+  // Whether steps run in one persistent kernel (run_kernel.cu) when the
+  // schedule is not fixed by hand.
+  bool use_whole_steps() const;
 
   // ---- adjoint (reverse-mode gradients of a trajectory; adjoint.cu) ----
   // Replaces the LJ eps/sigma tables of one replica (full n_types^2 tables).
@@ -217,6 +220,8 @@ class Engine {
   int4* relayout_img_ = nullptr;
   uint32_t* relayout_cross_ = nullptr;
   bool tuned_ = false;                 // autotune() has run
+  bool whole_steps_ = false;           // steps run in k_run (run_kernel.cu), not kernel by kernel
+  RunView run_{};                      // its work arrays
   cudaStream_t side_stream_ = nullptr;
   std::map<std::pair<uint32_t, bool>, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs_;
   std::map<uint32_t, std::pair<cudaGraph_t, cudaGraphExec_t>> replay_graphs_;

@@ -59,4 +59,27 @@ void launch_scatter_state(const StepLaunch& l, const float* pos_tag,
 void launch_gather_state(const StepLaunch& l, float* pos_tag, float* vel_tag,
                          uint32_t n_tags_total);
 
+
+// ---- whole steps in one kernel (run_kernel.cu) ----
+// Cross-block state of a launch; all zero between launches.
+struct RunControl {
+  uint32_t arrive;   // barrier arrivals of the launch
+  uint32_t left;     // blocks that have left it
+  uint32_t any[2];   // by step parity: some slot has moved half the skin
+  uint32_t reorder;  // some rebuilding replica reorders its slots
+};
+struct RunView {
+  RunControl* ctl;
+  uint32_t* work_atoms;  // [n_replicas + 1] particles of the rebuilding replicas before each
+  uint32_t* chunk_sum;   // [run_scan_chunks] cell-count totals
+  long long* ke_odd;     // kinetic-energy buckets of odd steps (even ones: DeviceView::ke_part)
+  int any_dense, any_sparse, need_kinetic;
+};
+constexpr int kRunBlocksPerSm = 7;  // resident blocks: the list build's registers
+// n_steps velocity-Verlet steps (observables: of the single step) or descent
+// iterations of every replica; slot-layout lists only.
+void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables);
+void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps);
+uint32_t run_scan_chunks(uint32_t total_cells);
+
 }  // namespace bb

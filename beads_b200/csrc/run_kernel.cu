@@ -1,0 +1,479 @@
+// run_kernel.cu -- whole MD steps in one persistent kernel.
+//
+// A step launched kernel by kernel costs about 28 us before any work: five
+// kernels at ~0.6 us each inside a captured graph, their own latencies, and
+// the conditional node that holds the rebuild chain (8 us when it is not
+// taken, 17 us when it is, on top of its kernels).  k_run takes a stretch of
+// steps instead: one cooperative launch of at most one wave of blocks, a
+// barrier over its blocks (1.1 us at up to 296 blocks, 1.3 us at 592) between
+// the stages, and the rebuild chain behind a flag every block reads after the
+// drift.  A step without a rebuild holds two barriers (three with bonded
+// terms), so it is bound by the latency of its own loads until the pair
+// forces fill the GPU.
+//
+// Every stage is the device function that the one-stage kernels call
+// (step_device.cuh), and the totals are integers, so a run gives the same
+// bits either way.  Blocks read positions and lists through the coherent path,
+// since the same kernel writes them.
+#include "kernels.cuh"
+#include "step_device.cuh"
+
+#include <algorithm>
+#include <stdexcept>
+#include <string>
+
+namespace bb {
+namespace {
+
+// One barrier over all blocks of the launch; `target` counts the arrivals of
+// this launch.  The wait is bounded: when the other blocks do not arrive
+// within some seconds it marks *status and returns false, and the caller
+// leaves the kernel.
+__device__ __forceinline__ bool grid_barrier(RunControl* ctl, unsigned* status,
+                                             uint32_t& target) {
+  __shared__ bool ok;
+  target += gridDim.x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // Release: the block's writes (ordered before this by the barrier above)
+    // are visible to whoever acquires the count.
+    uint32_t seen;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;"
+                 : "=r"(seen) : "l"(&ctl->arrive) : "memory");
+    bool done = static_cast<int32_t>(seen + 1u - target) >= 0;
+    for (uint32_t tries = 0; !done && tries < (1u << 23); ++tries) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&ctl->arrive) : "memory");
+      done = static_cast<int32_t>(seen - target) >= 0;
+    }
+    if (!done) atomicOr(status, kStatusStalled);
+    ok = done;
+  }
+  __syncthreads();
+  return ok;
+}
+
+union RunShared {
+  uint32_t sort_keys[kBlock / 32][kSortRankMax];
+  BuildShared build[kBuildWarps];
+};
+
+// Kinetic energy of replica r from its buckets (one full warp; lane 0 holds
+// the sum, like every other lane).
+__device__ __forceinline__ double bucket_kinetic(const long long* ke_part, uint32_t r,
+                                                 uint32_t lane) {
+  long long a = 0, c = 0;
+  const longlong2* bucket = reinterpret_cast<const longlong2*>(ke_part) + (size_t)r * kKeBuckets;
+#pragma unroll
+  for (uint32_t k = 0; k < kKeBuckets / 32u; ++k) {
+    const longlong2 q = __ldcg(&bucket[k * 32u + lane]);
+    a += q.x;
+    c += q.y;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(kFull, a, o);
+    c += __shfl_xor_sync(kFull, c, o);
+  }
+  return from_fixed(a, c);
+}
+
+// Runs F(v, b) for the listed slot blocks of the rebuilding replicas.
+template <typename F>
+__device__ __forceinline__ void for_listed_blocks(const DeviceView& v, F&& f) {
+  const uint32_t total = v.chain_block_start[v.n_replicas];
+  for (uint32_t w = blockIdx.x; w < total; w += gridDim.x) {
+    uint32_t lo = 0, hi = v.n_replicas;  // start[lo] <= w < start[hi]
+    while (hi - lo > 1u) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (v.chain_block_start[mid] <= w) lo = mid; else hi = mid;
+    }
+    f(v.rp[lo].block_begin + (w - v.chain_block_start[lo]));
+  }
+}
+
+constexpr uint32_t kMinGrid = 296;
+constexpr uint32_t kRunScanPer = 4;                        // consecutive cells per thread
+constexpr uint32_t kRunScanChunk = kBlock * kRunScanPer;  // work items per block of the scan
+
+// Rebuild decision of every replica and the work lists of the rebuilding ones
+// (block 0): work_start / chain_block_start / work_atoms hold the cells, slot
+// blocks and particles of the rebuilding replicas before each replica.
+// Steps since + 1 .. step - 1 of the launch moved no slot far enough; their
+// checks are counted here.
+__device__ __forceinline__ void count_checks(const ReplicaParams& p, ReplicaState* st,
+                                             uint32_t since, uint32_t step) {
+  if (p.skin == 0.0f || step <= since) return;
+  const unsigned long long lo = st->step + since, hi = st->step + step;
+  st->checks_since_build += p.check_every == 1u
+                                ? step - since
+                                : (uint32_t)(hi / p.check_every - lo / p.check_every);
+}
+
+template <int kPre>
+__device__ void run_decide(const DeviceView& v, const RunView& rv, uint32_t since,
+                           uint32_t step) {
+  uint32_t cells = 0, blocks = 0, atoms = 0, reorder = 0;
+  for (uint32_t base = 0; base < v.n_replicas; base += kBlock) {
+    const uint32_t r = base + threadIdx.x;
+    uint32_t c = 0, b = 0, n = 0;
+    bool move = false;
+    if (r < v.n_replicas) {
+      ReplicaState* st = &v.rs[r];
+      if (kPre == kPreVerlet) count_checks(v.rp[r], st, since, step);
+      if (decide_replica<kPre>(v.rp[r], st, st->step + step + 1ull)) {
+        c = v.rp[r].n_cells;
+        b = v.rp[r].n_pad / kBlock;
+        n = v.rp[r].n_atoms;
+        move = st->reorder_now != 0u;
+      }
+    }
+    uint32_t tc, tb, tn;
+    const uint32_t ec = block_exclusive_scan<kBlock>(c, tc);
+    const uint32_t eb = block_exclusive_scan<kBlock>(b, tb);
+    const uint32_t en = block_exclusive_scan<kBlock>(n, tn);
+    if (r < v.n_replicas) {
+      v.work_start[r] = cells + ec;
+      v.chain_block_start[r] = blocks + eb;
+      rv.work_atoms[r] = atoms + en;
+    }
+    cells += tc;
+    blocks += tb;
+    atoms += tn;
+    reorder |= __syncthreads_or(move ? 1 : 0);
+  }
+  if (threadIdx.x == 0) {
+    v.work_start[v.n_replicas] = cells;
+    v.chain_block_start[v.n_replicas] = blocks;
+    rv.work_atoms[v.n_replicas] = atoms;
+    rv.ctl->reorder = reorder;
+    if (cells != 0u) *v.chain_launches += 1ull;
+  }
+}
+
+// The rebuild chain of the replicas run_decide listed; false after a barrier
+// that ran out.
+__device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& rv,
+                                            RunShared& sh, uint32_t& target) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t items = v.work_start[v.n_replicas];
+  if (items == 0u) return true;  // launch-uniform
+  const bool reorder = rv.ctl->reorder != 0u;
+  for_listed_blocks(v, [&](uint32_t b) { bin_block(v, b); });
+  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  // Cell starts: totals of kRunScanChunk consecutive work items, then each
+  // chunk adds the totals before it.  Every particle of a rebuilding replica
+  // is counted once, so the running total of a replica's first cell is
+  // work_atoms.
+  const uint32_t chunks = (items + kRunScanChunk - 1u) / kRunScanChunk;
+  for (uint32_t ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
+    uint32_t s = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kRunScanPer; ++k) {
+      const uint32_t w = ch * kRunScanChunk + k * kBlock + threadIdx.x;
+      if (w < items) {
+        const uint32_t r = work_replica(v, w);
+        s += __ldcg(&v.cell_count[v.rp[r].cell_begin + (w - v.work_start[r])]);
+      }
+    }
+    uint32_t total;
+    block_exclusive_scan<kBlock>(s, total);
+    if (threadIdx.x == 0) rv.chunk_sum[ch] = total;
+  }
+  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  for (uint32_t ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
+    uint32_t before = 0;
+    for (uint32_t k = threadIdx.x; k < ch; k += kBlock) before += rv.chunk_sum[k];
+    uint32_t prefix;
+    block_exclusive_scan<kBlock>(before, prefix);
+    uint32_t cnt[kRunScanPer], s = 0;
+    const uint32_t w0 = ch * kRunScanChunk + threadIdx.x * kRunScanPer;
+#pragma unroll
+    for (uint32_t k = 0; k < kRunScanPer; ++k) {
+      cnt[k] = 0u;
+      if (w0 + k < items) {
+        const uint32_t r = work_replica(v, w0 + k);
+        cnt[k] = __ldcg(&v.cell_count[v.rp[r].cell_begin + (w0 + k - v.work_start[r])]);
+      }
+      s += cnt[k];
+    }
+    uint32_t total;
+    uint32_t run = prefix + block_exclusive_scan<kBlock>(s, total);
+#pragma unroll
+    for (uint32_t k = 0; k < kRunScanPer; ++k) {
+      if (w0 + k < items) {
+        const uint32_t r = work_replica(v, w0 + k);
+        const ReplicaParams& p = v.rp[r];
+        const uint32_t c = w0 + k - v.work_start[r];
+        const uint32_t at = p.atom_begin + run - rv.work_atoms[r];
+        v.cell_start[p.start_base + c] = at;
+        v.cell_cursor[p.cell_begin + c] = at;
+        v.cell_count[p.cell_begin + c] = 0u;
+        if (c + 1u == p.n_cells) v.cell_start[p.start_base + c + 1u] = p.atom_begin + p.n_atoms;
+      }
+      run += cnt[k];
+    }
+  }
+  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  for_listed_blocks(v, [&](uint32_t b) { scatter_block(v, b); });
+  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  if (rv.any_sparse) {
+    for (uint32_t w = blockIdx.x * kBlock + threadIdx.x; w < items; w += gridDim.x * kBlock) {
+      sort_cell_sparse(v, w);
+    }
+  }
+  for (uint32_t w = blockIdx.x * kBuildWarps + warp; w < items; w += gridDim.x * kBuildWarps) {
+    const uint32_t r = work_replica(v, w);
+    sort_cell(v, v.rp[r], w - v.work_start[r], lane, sh.sort_keys[warp]);
+    __syncwarp();
+  }
+  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  if (reorder) {
+    for_listed_blocks(v, [&](uint32_t b) { reorder_gather_block(v, b); });
+    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+    for_listed_blocks(v, [&](uint32_t b) { reorder_commit_block(v, b); });
+    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+    if (v.excl_cap > 0u) {
+      for_listed_blocks(v, [&](uint32_t b) { project_exclusions_block(v, b, false); });
+      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+    }
+  }
+  // A thread per particle only where sparse cells alone fill the GPU several
+  // times over: below that its serial walk of 27 cells (~60 us) is what the
+  // stage takes, and a warp per cell does the same lists in a fraction.
+  const uint32_t warps = gridDim.x * kBuildWarps;
+  const bool by_thread = rv.any_sparse && items > 24u * warps;
+  if (by_thread) {
+    // (slot rows: the stage layout is not touched)
+    for_listed_blocks(v, [&](uint32_t b) {
+      build_sparse_block<true, false>(v, b, sh.build[0].lay);
+    });
+  }
+  if (rv.any_dense || !by_thread) {
+    // A cell per warp, or a share of one.  A warp walks its cell's candidates
+    // in a few chunks (~1.5 us each) and its particles one by one within
+    // each (~0.25 us), so the share is chosen for the fewest such steps over
+    // the warps' rounds.
+    const uint32_t homes = rv.work_atoms[v.n_replicas] / items + 1u;
+    uint32_t parts = 1u, best = 0xffffffffu;
+    for (uint32_t t = 1u; t <= min(homes, 16u); ++t) {
+      const uint32_t rounds = (items * t + warps - 1u) / warps;
+      const uint32_t cost = rounds * (6u + (homes + t - 1u) / t);
+      if (cost < best) best = cost, parts = t;
+    }
+    for (uint32_t k = blockIdx.x * kBuildWarps + warp; k < items * parts; k += warps) {
+      const uint32_t w = k / parts;
+      const uint32_t r = work_replica(v, w);
+      const ReplicaParams& p = v.rp[r];
+      if (by_thread && p.sparse) continue;
+      build_cell<true, false>(v, p, &v.rs[r], p.cell_begin + (w - v.work_start[r]), lane,
+                              sh.build[warp], k - w * parts, parts);
+    }
+  }
+  return grid_barrier(rv.ctl, &v.rs->status, target);
+}
+
+// kPre: velocity Verlet (drift, rebuild, forces and second half-kick per step)
+// or the capped descent (forces, move, rebuild per iteration).  kObs: energies
+// and virial of the (single) step.
+template <int kPre, bool kObs, int kTpa, int kNt>
+__global__ void __launch_bounds__(kBlock, kRunBlocksPerSm)
+k_run(DeviceView v, RunView rv, uint32_t n_steps, float sd_dmax, float sd_fref) {
+  constexpr bool kVerlet = kPre == kPreVerlet;
+  __shared__ RunShared sh;
+  // The parameters and the LJ table of the replica at hand: after a barrier
+  // they would come from L2 again.
+  __shared__ ReplicaParams p;
+  __shared__ LjCoeff table[kNt == 0 ? kMaxTypes * kMaxTypes : kNt * kNt];
+  __shared__ float lam_s;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t gthread = blockIdx.x * kBlock + threadIdx.x;
+  const bool kinetic = kVerlet && (kObs || rv.need_kinetic != 0);
+  const bool bonded = v.has_bonded != 0;
+  uint32_t target = 0, cur = 0xffffffffu;
+  // Consecutive slot blocks and pair-force items per block: an item's
+  // neighbours are mostly those of the item before it.
+  const uint32_t b0 = (uint32_t)((uint64_t)v.n_blocks * blockIdx.x / gridDim.x);
+  const uint32_t b1 = (uint32_t)((uint64_t)v.n_blocks * (blockIdx.x + 1u) / gridDim.x);
+  const uint32_t n_items = v.n_blocks * kTpa;
+  const uint32_t i0 = (uint32_t)((uint64_t)n_items * blockIdx.x / gridDim.x);
+  const uint32_t i1 = (uint32_t)((uint64_t)n_items * (blockIdx.x + 1u) / gridDim.x);
+
+  auto enter = [&](uint32_t r) {  // block-uniform
+    if (r == cur) return;
+    cur = r;
+    __syncthreads();
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&v.rp[r]);
+    for (uint32_t k = threadIdx.x; k < sizeof(ReplicaParams) / 4u; k += kBlock) {
+      reinterpret_cast<uint32_t*>(&p)[k] = src[k];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < p.n_types * p.n_types; t += kBlock) {
+      table[t] = v.lj[p.lj_offset + t];
+    }
+    __syncthreads();
+  };
+  auto replica_of = [&](uint32_t b) -> uint32_t {
+    return v.n_replicas == 1u ? 0u : v.block_replica[b];
+  };
+
+  auto forces = [&](long long* ke) -> bool {
+    for (uint32_t item = i0; item < i1; ++item) {
+      enter(replica_of(item / kTpa));
+      lj_block<kObs, !kVerlet, kTpa, 4, true, kNt, true>(v, p, cur, item, table,
+                                                         kVerlet && !bonded, kinetic, ke);
+    }
+    if (bonded) {
+      const uint32_t terms = v.n_bond_terms + v.n_angle_terms + v.n_dihedral_terms;
+      for (uint32_t t = gthread; t < terms; t += gridDim.x * kBlock) bonded_term<kObs>(v, t);
+      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+      for (uint32_t b = b0; b < b1; ++b) {
+        enter(replica_of(b));
+        bonded_block<kObs>(v, p, cur, b, kVerlet, kinetic, ke);
+      }
+    }
+    return true;
+  };
+
+  uint32_t since = 0;  // steps whose checks are counted
+  for (uint32_t s = 0; s < n_steps; ++s) {
+    long long* ke = (s & 1u) ? rv.ke_odd : v.ke_part;
+    long long* ke_other = (s & 1u) ? v.ke_part : rv.ke_odd;
+    if (!kVerlet) {
+      if (!forces(nullptr)) return;
+      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+    }
+    uint32_t scaled = 0xffffffffu;
+    float lam = 1.0f;
+    for (uint32_t b = b0; b < b1; ++b) {
+      const uint32_t r = replica_of(b);
+      enter(r);
+      if (kVerlet && r != scaled && (s == 0u || (kinetic && p.thermostat == 1))) {
+        // The pending scale: the state's before the first step, then from
+        // the kinetic energy of the step before.
+        __syncthreads();
+        if (warp == 0) {
+          const double l =
+              s == 0u ? v.rs[r].lambda : berendsen_lambda(p, bucket_kinetic(ke_other, r, lane));
+          if (lane == 0u) lam_s = (float)l;
+        }
+        __syncthreads();
+        lam = lam_s;
+      } else if (r != scaled) {
+        lam = 1.0f;
+      }
+      scaled = r;
+      pre_block<kPre>(v, p, &v.rs[r], b, p.check_every == 1u ? 0ull : v.rs[r].step + s + 1ull, lam,
+                      sd_dmax, sd_fref, &rv.ctl->any[s & 1u]);
+      if (kVerlet && p.skin == 0.0f && threadIdx.x == 0) rv.ctl->any[s & 1u] = 1u;
+    }
+    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+    if (__ldcg(&rv.ctl->any[s & 1u]) != 0u) {  // launch-uniform
+      if (blockIdx.x == 0) run_decide<kPre>(v, rv, since, s);
+      since = s + 1u;
+      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+      if (!run_rebuild(v, rv, sh, target)) return;
+    }
+    // What follows is not read before the next barrier.
+    if (gthread == 0u) rv.ctl->any[(s + 1u) & 1u] = 0u;
+    if (kVerlet) {
+      if (kinetic) {
+        longlong2* z = reinterpret_cast<longlong2*>(ke_other);
+        for (uint32_t k = gthread; k < v.n_replicas * kKeBuckets; k += gridDim.x * kBlock) {
+          z[k] = make_longlong2(0, 0);
+        }
+      }
+      if (!forces(ke)) return;
+      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+    }
+  }
+  if (kVerlet) {
+    long long* ke = (n_steps & 1u) ? v.ke_part : rv.ke_odd;  // of the last step
+    for (uint32_t r = blockIdx.x * kBuildWarps + warp; r < v.n_replicas;
+         r += gridDim.x * kBuildWarps) {
+      double kin = 0.0;
+      if (kinetic) {
+        kin = bucket_kinetic(ke, r, lane);
+        longlong2* z = reinterpret_cast<longlong2*>(ke) + (size_t)r * kKeBuckets;
+        for (uint32_t k = lane; k < kKeBuckets; k += 32u) z[k] = make_longlong2(0, 0);
+      }
+      if (lane == 0u) {
+        ReplicaState* st = &v.rs[r];
+        if (since < n_steps) {
+          count_checks(v.rp[r], st, since, n_steps);
+          st->need_rebuild = 0u;
+          st->reorder_now = 0u;
+        }
+        finish_replica<kObs>(v, r, true, kinetic, n_steps, kin);
+      }
+    }
+  }
+  if (threadIdx.x == 0) {
+    if (blockIdx.x == 0) rv.ctl->any[0] = rv.ctl->any[1] = 0u;
+    __threadfence();
+    // The last block to leave rearms the barrier for the next launch.
+    if (atomicAdd(&rv.ctl->left, 1u) == gridDim.x - 1u) {
+      rv.ctl->arrive = 0u;
+      rv.ctl->left = 0u;
+    }
+  }
+}
+
+void check(cudaError_t e) {
+  if (e != cudaSuccess) {
+    throw std::runtime_error(std::string("CUDA launch of run failed: ") + cudaGetErrorString(e));
+  }
+}
+
+template <int kPre, bool kObs, int kTpa, int kNt>
+void launch_one(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
+  auto* kernel = k_run<kPre, kObs, kTpa, kNt>;
+  // One wave at most.  Pair-force items of a small system leave blocks idle,
+  // but a rebuild shares its cells over every warp, and barriers take the same
+  // time up to about two blocks per SM.
+  static const uint32_t wave = [&] {
+    int device = 0, sms = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) {
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, 0);
+    }
+    check(e);
+    return (uint32_t)(sms * per_sm);
+  }();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min(wave, std::max(kMinGrid, l.v.n_blocks * (uint32_t)kTpa)));
+  cfg.blockDim = dim3(kBlock);
+  cfg.stream = l.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  check(cudaLaunchKernelEx(&cfg, kernel, l.v, rv, n_steps, l.sd_dmax, l.sd_fref));
+}
+
+}  // namespace
+
+// Four threads per particle: a small system has threads to spare, and its
+// steps take as long as a thread's list.
+void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables) {
+  if (observables) {
+    launch_one<kPreVerlet, true, 4, 0>(l, rv, n_steps);
+  } else if (l.lj_types == 1) {
+    launch_one<kPreVerlet, false, 4, 1>(l, rv, n_steps);
+  } else if (l.lj_types == 2) {
+    launch_one<kPreVerlet, false, 4, 2>(l, rv, n_steps);
+  } else {
+    launch_one<kPreVerlet, false, 4, 0>(l, rv, n_steps);
+  }
+}
+
+void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
+  launch_one<kPreDescent, false, 4, 0>(l, rv, n_steps);
+}
+
+uint32_t run_scan_chunks(uint32_t total_cells) {
+  return (total_cells + kRunScanChunk - 1u) / kRunScanChunk;
+}
+
+}  // namespace bb
