@@ -149,12 +149,15 @@ bool Engine::use_whole_steps() const {
 void Engine::autotune() {
   TraceRange trace("beads.autotune");
   if (!initialized_) eval();
+  // The staged layout is kept only where it was asked for: the slot layout's
+  // global gathers mostly hit L1 and beat it on every size (1,048,576 beads:
+  // 0.174 against 0.233 ms a force evaluation).
+  if (v_.list_by_q != 0 && !layout_fixed_) {
+    v_.list_by_q = 0;
+    launch_.v = v_;
+    relayout_list();
+  }
   if (use_whole_steps()) {
-    if (v_.list_by_q != 0) {
-      v_.list_by_q = 0;
-      launch_.v = v_;
-      relayout_list();
-    }
     clear_graphs();
     whole_steps_ = true;
     launch_.lj_tpa = 4;
@@ -198,13 +201,10 @@ void Engine::autotune() {
   };
   // One coordinate at a time, each from the best so far: threads per
   // particle {1, 2, 4} at batch depth 4 with list loads bypassing L1, then
-  // depth 8, then list loads through L1 (the staged kernel reads its
-  // neighbour positions from shared memory and has no L1 choice), then the
-  // second half-kick fused into the force kernel: six trials per layout
-  // instead of the full grid of thirteen, which a short run pays for.
-  auto tune_layout = [&]() {
-    best = 0.f;
-    const bool staged_now = v_.list_by_q != 0;
+  // depth 8, then list loads through L1, then the second half-kick fused into
+  // the force kernel: six trials instead of the full grid of thirteen, which
+  // a short run pays for.
+  try {
     for (int tpa : {1, 2, 4}) {
       StepLaunch l = launch_;
       l.lj_tpa = tpa;
@@ -216,40 +216,12 @@ void Engine::autotune() {
     StepLaunch deeper = chosen;
     deeper.lj_unroll = 8;
     trial(deeper);
-    if (!staged_now) {
-      StepLaunch l1 = chosen;
-      l1.lj_no_l1 = 0;
-      trial(l1);
-    }
+    StepLaunch l1 = chosen;
+    l1.lj_no_l1 = 0;
+    trial(l1);
     StepLaunch fused = chosen;
     fused.fuse_post = 1;
     trial(fused);
-  };
-  try {
-    tune_layout();
-    // Both list layouts when the context can stage: the other layout is
-    // built from the same positions (relayout_list) and tuned the same way.
-    if (stage_cap_ > 0 && !layout_fixed_) {
-      const float best_first = best;
-      const StepLaunch chosen_first = chosen;
-      const bool first_staged = v_.list_by_q != 0;
-      v_.list_by_q = first_staged ? 0 : 1;
-      launch_.v = v_;
-      relayout_list();
-      tune_layout();
-      if (log) {
-        std::fprintf(stderr, "beads autotune: staged layout %.4f ms, slot layout %.4f ms\n",
-                     (first_staged ? best_first : best) / kReps,
-                     (first_staged ? best : best_first) / kReps);
-      }
-      if (best_first <= best) {
-        best = best_first;
-        chosen = chosen_first;
-        v_.list_by_q = first_staged ? 1 : 0;
-        launch_.v = v_;
-        relayout_list();
-      }
-    }
   } catch (...) {
     cudaEventDestroy(a);
     cudaEventDestroy(b);

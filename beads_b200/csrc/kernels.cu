@@ -413,8 +413,10 @@ k_lj(DeviceView v) {
 // entries reads global positions, as k_lj does.  The arithmetic, the list
 // order and the canonical summation order are k_lj's, so the forces, energies
 // and virial are bit-identical to k_lj's for the same list.
-template <bool kObs, int kMode, int kTpa, int kUnroll, bool kNoL1, int kNt>
+template <bool kObs, int kMode, int kTpa>
 __global__ void __launch_bounds__(kBlock* kTpa) k_lj_staged(DeviceView v) {
+  constexpr int kUnroll = 4, kNt = 0;  // the layout is kept for its bits, not its speed
+  constexpr bool kNoL1 = true;
   constexpr int kThreads = kBlock * kTpa;
   constexpr bool kClamp = kMode == kForceClamp;
   constexpr bool kPost = kMode >= kForcePost;
@@ -499,7 +501,7 @@ __global__ void __launch_bounds__(kBlock* kTpa) k_lj_staged(DeviceView v) {
   double ke = 0.0;
   if (kPost) ke = post_slot_vm(v, p, st, i, owner, true, kKinetic, vm_kick, fx, fy, fz);
   if (kObs) {
-    const float e = ae.total(), w = aw.total();
+    const float e = ae.total(), w = -aw.total();
     block_add_lane<kThreads>(owner, 0.5 * (double)e, st, kAccPair);
     block_add_lane<kThreads>(owner, 0.5 * (double)w, st, kAccVirial);
   }
@@ -785,74 +787,52 @@ namespace {
 // shared memory.
 size_t staged_smem(const StepLaunch& l) { return (size_t)(l.v.stage_cap + 1u) * sizeof(float4); }
 
-template <bool kObs, int kMode, int kTpa, int kUnroll, int kNt>
+template <bool kObs, int kMode, int kTpa>
 void staged_one(const StepLaunch& l) {
-  k_lj_staged<kObs, kMode, kTpa, kUnroll, true, kNt>
-      <<<l.v.n_blocks, kBlock * kTpa, staged_smem(l), l.stream>>>(l.v);
+  k_lj_staged<kObs, kMode, kTpa><<<l.v.n_blocks, kBlock * kTpa, staged_smem(l), l.stream>>>(l.v);
 }
 
-template <bool kObs, int kMode, int kTpa, int kUnroll, int kNt>
+template <bool kObs, int kMode, int kTpa>
 void staged_attr(size_t smem) {
-  const cudaError_t e =
-      cudaFuncSetAttribute(k_lj_staged<kObs, kMode, kTpa, kUnroll, true, kNt>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = cudaFuncSetAttribute(k_lj_staged<kObs, kMode, kTpa>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     throw std::runtime_error(std::string("staged pair kernel shared memory: ") +
                              cudaGetErrorString(e));
   }
 }
 
-template <int kTpa, int kUnroll, int kNt>
-void staged_attr_modes(size_t smem) {
-  staged_attr<false, kForcePlain, kTpa, kUnroll, kNt>(smem);
-  staged_attr<false, kForcePost, kTpa, kUnroll, kNt>(smem);
-  staged_attr<false, kForcePostKinetic, kTpa, kUnroll, kNt>(smem);
+template <int kTpa>
+void staged_attrs(size_t smem) {
+  staged_attr<true, kForcePlain, kTpa>(smem);
+  staged_attr<true, kForcePost, kTpa>(smem);
+  staged_attr<false, kForcePlain, kTpa>(smem);
+  staged_attr<false, kForcePost, kTpa>(smem);
+  staged_attr<false, kForcePostKinetic, kTpa>(smem);
 }
 
-template <int kTpa, int kUnroll, int kNt>
-void staged_plain(const StepLaunch& l, int mode) {
-  switch (mode) {
-    case kForcePlain: staged_one<false, kForcePlain, kTpa, kUnroll, kNt>(l); break;
-    case kForcePost: staged_one<false, kForcePost, kTpa, kUnroll, kNt>(l); break;
-    default: staged_one<false, kForcePostKinetic, kTpa, kUnroll, kNt>(l); break;
-  }
-}
-
-template <int kTpa, int kUnroll>
-void staged_plain_nt(const StepLaunch& l, int mode) {
-  switch (l.lj_types) {
-    case 1: staged_plain<kTpa, kUnroll, 1>(l, mode); break;
-    case 2: staged_plain<kTpa, kUnroll, 2>(l, mode); break;
-    default: staged_plain<kTpa, kUnroll, 0>(l, mode); break;
+template <int kTpa>
+void launch_staged(const StepLaunch& l, bool observables, int mode) {
+  if (observables) {
+    if (mode == kForcePlain) staged_one<true, kForcePlain, kTpa>(l);
+    else staged_one<true, kForcePost, kTpa>(l);
+  } else {
+    switch (mode) {
+      case kForcePlain: staged_one<false, kForcePlain, kTpa>(l); break;
+      case kForcePost: staged_one<false, kForcePost, kTpa>(l); break;
+      default: staged_one<false, kForcePostKinetic, kTpa>(l); break;
+    }
   }
 }
 
 void launch_forces_staged(const StepLaunch& l, bool observables, bool clamp, int mode) {
   if (clamp) {
-    staged_one<false, kForceClamp, 2, 4, 0>(l);
-  } else if (observables) {
-    const bool plain = mode == kForcePlain;
-    switch (l.lj_tpa) {
-      case 2:
-        plain ? staged_one<true, kForcePlain, 2, 4, 0>(l) : staged_one<true, kForcePost, 2, 4, 0>(l);
-        break;
-      case 4:
-        plain ? staged_one<true, kForcePlain, 4, 4, 0>(l) : staged_one<true, kForcePost, 4, 4, 0>(l);
-        break;
-      default:
-        plain ? staged_one<true, kForcePlain, 1, 4, 0>(l) : staged_one<true, kForcePost, 1, 4, 0>(l);
-        break;
-    }
+    staged_one<false, kForceClamp, 2>(l);
   } else {
-    const int key = l.lj_tpa * 10 + l.lj_unroll;
-    switch (key) {
-      case 14: staged_plain_nt<1, 4>(l, mode); break;
-      case 18: staged_plain_nt<1, 8>(l, mode); break;
-      case 24: staged_plain_nt<2, 4>(l, mode); break;
-      case 28: staged_plain_nt<2, 8>(l, mode); break;
-      case 44: staged_plain_nt<4, 4>(l, mode); break;
-      case 48: staged_plain_nt<4, 8>(l, mode); break;
-      default: throw std::runtime_error("unsupported staged pair-force schedule");
+    switch (l.lj_tpa) {
+      case 2: launch_staged<2>(l, observables, mode); break;
+      case 4: launch_staged<4>(l, observables, mode); break;
+      default: launch_staged<1>(l, observables, mode); break;
     }
   }
   check_launch("lj_staged");
@@ -863,19 +843,10 @@ void launch_forces_staged(const StepLaunch& l, bool observables, bool clamp, int
 // Raises the dynamic shared-memory limit of every staged pair-force variant to
 // `smem` bytes (once per context, outside any stream capture).
 void prepare_staged_kernels(size_t smem) {
-  staged_attr<false, kForceClamp, 2, 4, 0>(smem);
-  staged_attr<true, kForcePlain, 1, 4, 0>(smem);
-  staged_attr<true, kForcePost, 1, 4, 0>(smem);
-  staged_attr<true, kForcePlain, 2, 4, 0>(smem);
-  staged_attr<true, kForcePost, 2, 4, 0>(smem);
-  staged_attr<true, kForcePlain, 4, 4, 0>(smem);
-  staged_attr<true, kForcePost, 4, 4, 0>(smem);
-#define BB_ATTR(t, u)                    \
-  staged_attr_modes<t, u, 0>(smem);      \
-  staged_attr_modes<t, u, 1>(smem);      \
-  staged_attr_modes<t, u, 2>(smem);
-  BB_ATTR(1, 4) BB_ATTR(1, 8) BB_ATTR(2, 4) BB_ATTR(2, 8) BB_ATTR(4, 4) BB_ATTR(4, 8)
-#undef BB_ATTR
+  staged_attr<false, kForceClamp, 2>(smem);
+  staged_attrs<1>(smem);
+  staged_attrs<2>(smem);
+  staged_attrs<4>(smem);
 }
 
 void launch_list_to_slots(const StepLaunch& l, uint32_t cap, uint32_t* out_count, uint32_t* out) {

@@ -1085,6 +1085,13 @@ __device__ __forceinline__ uint32_t list_load(const uint32_t* p) {
   return __ldcs(p);
 }
 
+// 1 / x for x in the range of squared distances (denormals flushed).
+__device__ __forceinline__ float reciprocal(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // LJ coefficients of two pairs as packed pairs.  kNt = 1 (every replica has
 // one particle type): the row is held in registers and already packed;
 // kNt = 2: the particle's two-entry row in registers, selected by the
@@ -1151,9 +1158,9 @@ __device__ __forceinline__ void lj_pairs(const DeviceView& v, const ReplicaParam
                                          uint32_t sub, uint32_t n, uint32_t n_warp, float rc2,
                                          float half_min_sq, LjAcc<kTpa>& ax, LjAcc<kTpa>& ay,
                                          LjAcc<kTpa>& az, LjAcc<kTpa>& ae, LjAcc<kTpa>& aw) {
-  const float2 xi2x = make_float2(xi.x, xi.x);
-  const float2 xi2y = make_float2(xi.y, xi.y);
-  const float2 xi2z = make_float2(xi.z, xi.z);
+  const float2 nxi = make_float2(-xi.x, -xi.x);
+  const float2 nyi = make_float2(-xi.y, -xi.y);
+  const float2 nzi = make_float2(-xi.z, -xi.z);
   const uint32_t* list = v.nbr + nbr_index(row, 0, v.nbr_stride) + sub * kGroup;
   // Software-pipelined over batches of kUnroll (4 or 8) own entries: all
   // list loads of a batch are issued, then all position gathers, then the
@@ -1192,9 +1199,11 @@ __device__ __forceinline__ void lj_pairs(const DeviceView& v, const ReplicaParam
 #pragma unroll
     for (uint32_t h = 0; h < kUnroll / 2; ++h) {
       const uint32_t u0 = 2 * h, u1 = 2 * h + 1;
-      float2 dx = __fadd2_rn(xi2x, make_float2(-xj[u0].x, -xj[u1].x));
-      float2 dy = __fadd2_rn(xi2y, make_float2(-xj[u0].y, -xj[u1].y));
-      float2 dz = __fadd2_rn(xi2z, make_float2(-xj[u0].z, -xj[u1].z));
+      // Neighbour minus particle: no negation of the gathered coordinates
+      // (the force scale below carries the sign; the bits are the same).
+      float2 dx = __fadd2_rn(make_float2(xj[u0].x, xj[u1].x), nxi);
+      float2 dy = __fadd2_rn(make_float2(xj[u0].y, xj[u1].y), nyi);
+      float2 dz = __fadd2_rn(make_float2(xj[u0].z, xj[u1].z), nzi);
       float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
       // Plain differences are already the once-rounded exact values unless
       // the pair straddles the periodic boundary, which needs r^2 above
@@ -1206,12 +1215,9 @@ __device__ __forceinline__ void lj_pairs(const DeviceView& v, const ReplicaParam
         // Both pairs at once through the packed pipe, each lane rounded
         // exactly as acc_delta / norm2 round it; pairs that are not far keep
         // their plain differences.
-        dx = acc_delta2(dx, xi2x, make_float2(-xj[u0].x, -xj[u1].x), p.len[0], p.half[0],
-                        far0, far1);
-        dy = acc_delta2(dy, xi2y, make_float2(-xj[u0].y, -xj[u1].y), p.len[1], p.half[1],
-                        far0, far1);
-        dz = acc_delta2(dz, xi2z, make_float2(-xj[u0].z, -xj[u1].z), p.len[2], p.half[2],
-                        far0, far1);
+        dx = acc_delta2(dx, make_float2(xj[u0].x, xj[u1].x), nxi, p.len[0], p.half[0], far0, far1);
+        dy = acc_delta2(dy, make_float2(xj[u0].y, xj[u1].y), nyi, p.len[1], p.half[1], far0, far1);
+        dz = acc_delta2(dz, make_float2(xj[u0].z, xj[u1].z), nzi, p.len[2], p.half[2], far0, far1);
         const float2 r2f = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
         r2 = make_float2(far0 ? r2f.x : r2.x, far1 ? r2f.y : r2.y);
       }
@@ -1227,20 +1233,21 @@ __device__ __forceinline__ void lj_pairs(const DeviceView& v, const ReplicaParam
         rr.x = fmaxf(rr.x, 0.49f * c.sigma2.x);
         rr.y = fmaxf(rr.y, 0.49f * c.sigma2.y);
       }
-      const float2 inv = make_float2(__fdividef(1.0f, rr.x), __fdividef(1.0f, rr.y));
+      const float2 inv = make_float2(reciprocal(rr.x), reciprocal(rr.y));
       const float2 sr2 = __fmul2_rn(c.sigma2, inv);
       const float2 sr6 = __fmul2_rn(__fmul2_rn(sr2, sr2), sr2);
       const float2 sr12 = __fmul2_rn(sr6, sr6);
-      const float2 neg6 = make_float2(-sr6.x, -sr6.y);
-      const float2 g = __ffma2_rn(make_float2(2.0f, 2.0f), sr12, neg6);
-      float2 fs = __fmul2_rn(__fmul2_rn(c.eps24, inv), g);
+      // Minus the force scale, against the minus of the differences.
+      const float2 g = __ffma2_rn(make_float2(-2.0f, -2.0f), sr12, sr6);
+      const float2 fs = __fmul2_rn(__fmul2_rn(c.eps24, inv), g);
       ax.add_fma(h, fs, dx);
       ay.add_fma(h, fs, dy);
       az.add_fma(h, fs, dz);
       if (kObs) {
-        const float2 ep = __ffma2_rn(c.eps4, __fadd2_rn(sr12, neg6), c.neg_shift);
+        const float2 e = __fadd2_rn(sr12, make_float2(-sr6.x, -sr6.y));
+        const float2 ep = __ffma2_rn(c.eps4, e, c.neg_shift);
         ae.add(h, make_float2(in0 ? ep.x : 0.0f, in1 ? ep.y : 0.0f));
-        aw.add_fma(h, fs, rr);
+        aw.add_fma(h, fs, rr);  // minus the virial
       }
     }
   }
@@ -1308,7 +1315,7 @@ __device__ __forceinline__ void lj_block(const DeviceView& v, const ReplicaParam
   double ke = 0.0;
   if (post) ke = post_slot_vm(v, p, st, i, owner, true, kinetic, vm_kick, fx, fy, fz);
   if (kObs) {
-    const float e = ae.total(), w = aw.total();
+    const float e = ae.total(), w = -aw.total();
     block_add_lane<kBlock>(owner, 0.5 * (double)e, st, kAccPair);
     block_add_lane<kBlock>(owner, 0.5 * (double)w, st, kAccVirial);
   }
