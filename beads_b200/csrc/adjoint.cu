@@ -36,6 +36,7 @@
 #include "device_util.cuh"
 #include "engine.hpp"
 #include "kernels.cuh"
+#include "step_device.cuh"
 #include "trace.hpp"
 
 namespace bb {
@@ -111,25 +112,14 @@ __global__ void k_adj_list_positions(DeviceView v, AdjView a, uint32_t segment,
                      : a.seg_pos[(size_t)src * a.slots + i];
 }
 
-// Copies the list rows (and counts) of slot block b into snapshot k: every
-// block when `all`, else the blocks of replicas that rebuilt their list in
-// the step just run.  A block's 128 rows are one contiguous run of the
-// interleaved list (4 whole groups of 32 rows).
-__global__ void k_adj_snapshot(DeviceView v, uint32_t* snap_nbr, uint32_t* snap_cnt,
-                               uint32_t k, int all) {
+// Snapshot k of the list: every block when `all`, else the blocks of replicas
+// that rebuilt their list in the step just run.
+__global__ void __launch_bounds__(kBlock)
+k_adj_snapshot(DeviceView v, uint32_t* snap_nbr, uint32_t* snap_cnt, uint32_t k, int all) {
   const uint32_t b = blockIdx.x;
-  const uint32_t r = v.block_replica[b];
-  if (!all && !v.rs[r].need_rebuild) return;
-  const size_t entries = (size_t)kBlock * v.nbr_stride;
-  const size_t base = (size_t)b * entries;
-  const size_t per_snap = (size_t)v.n_slots * v.nbr_stride;
-  const uint4* src = reinterpret_cast<const uint4*>(v.nbr + base);
-  uint4* dst = reinterpret_cast<uint4*>(snap_nbr + (size_t)k * per_snap + base);
-  for (size_t t = threadIdx.x; t < entries / 4; t += blockDim.x) dst[t] = __ldcs(src + t);
-  if (threadIdx.x < kBlock) {
-    const size_t i = (size_t)b * kBlock + threadIdx.x;
-    snap_cnt[(size_t)k * v.n_slots + i] = v.nbr_count[i];
-  }
+  if (!all && !v.rs[v.block_replica[b]].need_rebuild) return;
+  const size_t at = (size_t)k * v.n_slots;
+  snapshot_block(v, b, snap_nbr + at * v.nbr_stride, snap_cnt + at);
 }
 
 // Crossing counts of restored slots: img - ref_img of the checkpoint.
@@ -626,7 +616,6 @@ void Engine::set_lj(uint32_t replica, const double* eps, const double* sigma) {
       table[static_cast<size_t>(i) * nt + j] = c;
     }
   }
-  sync();
   h2d(const_cast<LjCoeff*>(v_.lj) + h.lj_offset, table.data(), table.size() * sizeof(LjCoeff),
       "LJ table upload");
   initialized_ = false;  // forces of the current state are stale
@@ -697,12 +686,28 @@ void Engine::adjoint_record(uint32_t k) {
   launch_check("adjoint record");
 }
 
+// The segment store as the record of a k_run launch that takes the steps after
+// record k0.
+RunRecord Engine::adjoint_run_record(uint32_t k0) {
+  AdjointStore& A = *adj_;
+  RunRecord rec{};
+  rec.pos = A.seg_pos;
+  rec.vel = A.seg_vel;
+  rec.lam = A.seg_lam;
+  rec.kin = A.seg_kin;
+  rec.flags = A.seg_flags;
+  rec.snap_nbr = A.snap_on ? A.snap_nbr : nullptr;
+  rec.snap_cnt = A.snap_on ? A.snap_cnt : nullptr;
+  rec.k0 = k0;
+  return rec;
+}
+
 // Snapshot k of the list (see k_adj_snapshot); nothing when the backward
 // pass rebuilds its lists instead.
 void Engine::adjoint_snapshot(uint32_t k, bool all) {
   AdjointStore& A = *adj_;
   if (!A.snap_on) return;
-  k_adj_snapshot<<<v_.n_blocks, 256, 0, stream_>>>(v_, A.snap_nbr, A.snap_cnt, k, all ? 1 : 0);
+  k_adj_snapshot<<<v_.n_blocks, kBlock, 0, stream_>>>(v_, A.snap_nbr, A.snap_cnt, k, all ? 1 : 0);
   launch_check("adjoint list snapshot");
 }
 
@@ -803,8 +808,7 @@ void Engine::adjoint_forward(uint64_t steps, uint64_t record_from, uint32_t ever
     d2h(A.ck_state.data() + static_cast<size_t>(c) * R, v_.rs, R * sizeof(ReplicaState), "checkpoint");
   };
   std::vector<beads_observables> o;
-  auto put_obs = [&](uint64_t n) {
-    observables(o);
+  auto write_obs = [&](uint64_t n) {
     for (uint32_t r = 0; r < R; ++r) {
       double* row = obs + ((n - record_from) * R + r) * 3;
       row[0] = o[r].pe;
@@ -812,9 +816,19 @@ void Engine::adjoint_forward(uint64_t steps, uint64_t record_from, uint32_t ever
       row[2] = o[r].ke;
     }
   };
+  auto put_obs = [&](uint64_t n) {
+    observables(o);
+    write_obs(n);
+  };
 
   eval();
   if (!tuned_ && !tuning_fixed_) autotune();
+  // Whole steps: the recorded window runs in launches of up to kObsRing steps
+  // that keep every step's observables (and, storing every step, its state) on
+  // the device.
+  constexpr uint64_t kObsRing = 64;
+  std::vector<ReplicaObs> ring;
+  if (whole_steps_ && !A.obs_ring) A.obs_ring = A.alloc<ReplicaObs>(kObsRing * R);
   save(0);
   if (record_from == 0) put_obs(0);
   if (A.store_all) {
@@ -824,7 +838,31 @@ void Engine::adjoint_forward(uint64_t steps, uint64_t record_from, uint32_t ever
   uint64_t n = 0;
   while (n < steps) {
     const uint64_t next_ck = (n / every + 1) * every;
-    if (A.store_all) {
+    if (whole_steps_ && (A.store_all || n + 1 >= record_from)) {
+      const bool observe = n + 1 >= record_from;
+      const uint64_t m = std::min({next_ck - n, observe ? steps - n : record_from - 1 - n,
+                                   steps - n, kObsRing});
+      RunRecord rec{};
+      if (A.store_all) {
+        rec = adjoint_run_record(static_cast<uint32_t>(n));
+        rec.snap_nbr = rec.snap_cnt = nullptr;
+        cuda_check(cudaMemsetAsync(A.seg_flags + (n + 1) * R, 0, m * R * sizeof(uint32_t), stream_),
+                   "memset");
+      }
+      rec.obs = A.obs_ring;
+      launch_run(launch_, run_, static_cast<uint32_t>(m), observe, rec);
+      step_ += m;
+      if (observe) {
+        ring.resize(m * R);
+        d2h(ring.data(), A.obs_ring, ring.size() * sizeof(ReplicaObs), "observables download");
+        for (uint64_t k = 0; k < m; ++k) {
+          convert_observables(ring.data() + k * R, o);
+          write_obs(n + 1 + k);
+        }
+      }
+      check_status();
+      n += m;
+    } else if (A.store_all) {
       run(1, n + 1 >= record_from ? 1 : 0);
       n += 1;
       adjoint_record(static_cast<uint32_t>(n));
@@ -959,7 +997,17 @@ void Engine::adjoint_backward(const double* obs_grad, double* grad_eps, double* 
     // when it stored every step).
     if (!A.store_all) {
       adjoint_restore(static_cast<uint32_t>(s));
-      if (use_graphs_) {
+      if (whole_steps_) {
+        adjoint_record(0);
+        adjoint_snapshot(0, true);
+        cuda_check(cudaMemsetAsync(A.seg_flags + R, 0, static_cast<size_t>(b - a) * R *
+                   sizeof(uint32_t), stream_), "memset");
+        constexpr uint64_t kReplayChunk = 256;
+        for (uint64_t k = 0; k < b - a; k += kReplayChunk) {
+          launch_run(launch_, run_, static_cast<uint32_t>(std::min(kReplayChunk, b - a - k)), false,
+                     adjoint_run_record(static_cast<uint32_t>(k)));
+        }
+      } else if (use_graphs_) {
         cuda_check(cudaGraphLaunch(replay_graph_for(static_cast<uint32_t>(b - a)), stream_),
                    "replay launch");
       } else {

@@ -73,6 +73,8 @@ struct AdjointStore {
   long long* theta_angle = nullptr;  // [angle types][k, theta0][2]
   long long* theta_dihedral = nullptr;  // [dihedral types][2]
 
+  ReplicaObs* obs_ring = nullptr;  // [64][R] observables of the steps of one launch
+
   std::vector<void*> allocations;
   ~AdjointStore();
   template <typename T>

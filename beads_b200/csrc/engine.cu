@@ -78,12 +78,14 @@ Engine::Engine(uint32_t n, const beads_system_desc* systems,
 }
 
 void Engine::set_sort_enabled(bool on) {
+  // One strided copy of every replica's cadence.
+  std::vector<uint32_t> value(rep_.size(), 0u);
+  for (uint32_t r = 0; on && r < rep_.size(); ++r) value[r] = rep_[r].sort_every;
+  ReplicaParams* dst = const_cast<ReplicaParams*>(v_.rp);
+  cuda_check(cudaMemcpy2DAsync(&dst->sort_every, sizeof(ReplicaParams), value.data(),
+                               sizeof(uint32_t), sizeof(uint32_t), value.size(),
+                               cudaMemcpyHostToDevice, stream_), "sort cadence");
   sync();
-  for (uint32_t r = 0; r < rep_.size(); ++r) {
-    const uint32_t value = on ? rep_[r].sort_every : 0u;
-    ReplicaParams* dst = const_cast<ReplicaParams*>(v_.rp) + r;
-    h2d(&dst->sort_every, &value, sizeof(value), "sort cadence");
-  }
 }
 
 void Engine::clear_graphs() {
@@ -1164,9 +1166,13 @@ void Engine::list_stats(uint64_t* total, uint32_t* max_count) {
 void Engine::observables(std::vector<beads_observables>& out) {
   sync();
   d2h(h_obs_, v_.obs, rep_.size() * sizeof(ReplicaObs), "observables download");
+  convert_observables(h_obs_, out);
+}
+
+void Engine::convert_observables(const ReplicaObs* raw, std::vector<beads_observables>& out) const {
   out.resize(rep_.size());
   for (uint32_t r = 0; r < rep_.size(); ++r) {
-    const ReplicaObs& o = h_obs_[r];
+    const ReplicaObs& o = raw[r];
     const ReplicaHost& h = rep_[r];
     beads_observables& b = out[r];
     b.step = o.step;

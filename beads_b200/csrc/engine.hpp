@@ -87,6 +87,7 @@ class Engine {
   void minimize(uint32_t iterations, float dmax, float fref);
 
   void observables(std::vector<beads_observables>& out);
+  void convert_observables(const ReplicaObs* raw, std::vector<beads_observables>& out) const;
   void state(uint32_t r, float* pos, float* vel, float* force, int32_t* img,
              uint32_t* tag_slot_order = nullptr, int32_t* type_slot = nullptr);
   // Slot-order view of one replica (for trajectory records / snapshots).
@@ -173,6 +174,7 @@ class Engine {
   void adjoint_restore(uint32_t segment);
   void adjoint_record(uint32_t k);
   void adjoint_snapshot(uint32_t k, bool all);
+  RunRecord adjoint_run_record(uint32_t k0);
   void adjoint_segment_storage(uint32_t K);
   void adjoint_select_list(uint32_t a, uint32_t m, std::vector<int>& current,
                            const std::vector<uint32_t>& flags);

@@ -38,7 +38,7 @@ k_pre(DeviceView v, float sd_dmax, float sd_fref) {
   const uint32_t r = v.block_replica[blockIdx.x];
   ReplicaState* st = &v.rs[r];
   pre_block<kMode>(v, v.rp[r], st, blockIdx.x, st->step + 1ull,
-                   (kMode == kPreVerlet) ? (float)st->lambda : 1.0f, sd_dmax, sd_fref, nullptr);
+                   (kMode == kPreVerlet) ? (float)st->lambda : 1.0f, sd_dmax, sd_fref, nullptr, nullptr);
 }
 
 // pre, second part: one thread per replica takes the rebuild decision of
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_post_finish(DeviceView v) {
     }
     kin = from_fixed(sa, sc);
   }
-  finish_replica<kObs>(v, r, kKick, kKinetic, 1ull, kin);
+  finish_replica<kObs>(v, r, kKick, kKinetic, kin);
 }
 
 template <bool kObs, int kMode, int kTpa, int kUnroll, bool kNoL1, int kNt>

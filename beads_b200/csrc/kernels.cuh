@@ -75,10 +75,27 @@ struct RunView {
   long long* ke_odd;     // kinetic-energy buckets of odd steps (even ones: DeviceView::ke_part)
   int any_dense, any_sparse, need_kinetic;
 };
+// What a launch of k_run records of its steps (every pointer may be null).
+// Step s of the launch (0-based) writes record k0 + s + 1: positions and
+// velocities per slot, pending Berendsen scale, kinetic energy and rebuild
+// flag per replica, and the list rows of the replicas that rebuilt.
+struct RunRecord {
+  float4* pos;         // [record][n_slots]
+  float4* vel;
+  double* lam;         // [record][n_replicas]
+  double* kin;
+  uint32_t* flags;     // zero where no replica rebuilds
+  uint32_t* snap_nbr;  // [record][n_slots * nbr_stride]
+  uint32_t* snap_cnt;  // [record][n_slots]
+  uint32_t k0;
+  ReplicaObs* obs;     // [step of the launch][n_replicas] (launches with observables)
+};
 constexpr int kRunBlocksPerSm = 7;  // resident blocks: the list build's registers
-// n_steps velocity-Verlet steps (observables: of the single step) or descent
-// iterations of every replica; slot-layout lists only.
-void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables);
+// n_steps velocity-Verlet steps or descent iterations of every replica;
+// slot-layout lists only.  observables: energies and virial of every step
+// (DeviceView::obs keeps the last step's).
+void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables,
+                const RunRecord& rec = RunRecord{});
 void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps);
 uint32_t run_scan_chunks(uint32_t total_cells);
 

@@ -110,8 +110,8 @@ __device__ __forceinline__ void count_checks(const ReplicaParams& p, ReplicaStat
 }
 
 template <int kPre>
-__device__ void run_decide(const DeviceView& v, const RunView& rv, uint32_t since,
-                           uint32_t step) {
+__device__ void run_decide(const DeviceView& v, const RunView& rv, const RunRecord& rec,
+                           uint32_t since, uint32_t step) {
   uint32_t cells = 0, blocks = 0, atoms = 0, reorder = 0;
   for (uint32_t base = 0; base < v.n_replicas; base += kBlock) {
     const uint32_t r = base + threadIdx.x;
@@ -125,6 +125,7 @@ __device__ void run_decide(const DeviceView& v, const RunView& rv, uint32_t sinc
         b = v.rp[r].n_pad / kBlock;
         n = v.rp[r].n_atoms;
         move = st->reorder_now != 0u;
+        if (rec.flags) rec.flags[(size_t)(rec.k0 + step + 1u) * v.n_replicas + r] = 1u;
       }
     }
     uint32_t tc, tb, tn;
@@ -274,10 +275,10 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
 
 // kPre: velocity Verlet (drift, rebuild, forces and second half-kick per step)
 // or the capped descent (forces, move, rebuild per iteration).  kObs: energies
-// and virial of the (single) step.
+// and virial of every step.
 template <int kPre, bool kObs, int kTpa, int kNt>
 __global__ void __launch_bounds__(kBlock, kRunBlocksPerSm)
-k_run(DeviceView v, RunView rv, uint32_t n_steps, float sd_dmax, float sd_fref) {
+k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, float sd_fref) {
   constexpr bool kVerlet = kPre == kPreVerlet;
   __shared__ RunShared sh;
   // The parameters and the LJ table of the replica at hand: after a barrier
@@ -316,11 +317,11 @@ k_run(DeviceView v, RunView rv, uint32_t n_steps, float sd_dmax, float sd_fref) 
     return v.n_replicas == 1u ? 0u : v.block_replica[b];
   };
 
-  auto forces = [&](long long* ke) -> bool {
+  auto forces = [&](long long* ke, float4* vel) -> bool {
     for (uint32_t item = i0; item < i1; ++item) {
       enter(replica_of(item / kTpa));
       lj_block<kObs, !kVerlet, kTpa, 4, true, kNt, true>(v, p, cur, item, table,
-                                                         kVerlet && !bonded, kinetic, ke);
+                                                         kVerlet && !bonded, kinetic, ke, vel);
     }
     if (bonded) {
       const uint32_t terms = v.n_bond_terms + v.n_angle_terms + v.n_dihedral_terms;
@@ -328,10 +329,30 @@ k_run(DeviceView v, RunView rv, uint32_t n_steps, float sd_dmax, float sd_fref) 
       if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
       for (uint32_t b = b0; b < b1; ++b) {
         enter(replica_of(b));
-        bonded_block<kObs>(v, p, cur, b, kVerlet, kinetic, ke);
+        bonded_block<kObs>(v, p, cur, b, kVerlet, kinetic, ke, vel);
       }
     }
     return true;
+  };
+
+  // What step s left, replica by replica (a warp each), once its buckets are
+  // complete: observables and recorded scale and kinetic energy.
+  auto epilogue = [&](uint32_t s, const long long* ke) {
+    for (uint32_t r = blockIdx.x * kBuildWarps + warp; r < v.n_replicas;
+         r += gridDim.x * kBuildWarps) {
+      const double kin = kinetic ? bucket_kinetic(ke, r, lane) : 0.0;
+      if (lane != 0u) continue;
+      const double l = kinetic ? berendsen_lambda(v.rp[r], kin) : 1.0;
+      if (rec.lam) {
+        rec.lam[(size_t)(rec.k0 + s + 1u) * v.n_replicas + r] = l;
+        rec.kin[(size_t)(rec.k0 + s + 1u) * v.n_replicas + r] = kin;
+      }
+      if (kObs) {
+        const ReplicaObs o = take_observables(&v.rs[r], v.rs[r].step + s + 1ull, kin, l);
+        if (rec.obs) rec.obs[(size_t)s * v.n_replicas + r] = o;
+        if (s + 1u == n_steps) v.obs[r] = o;
+      }
+    }
   };
 
   uint32_t since = 0;  // steps whose checks are counted
@@ -339,9 +360,11 @@ k_run(DeviceView v, RunView rv, uint32_t n_steps, float sd_dmax, float sd_fref) 
     long long* ke = (s & 1u) ? rv.ke_odd : v.ke_part;
     long long* ke_other = (s & 1u) ? v.ke_part : rv.ke_odd;
     if (!kVerlet) {
-      if (!forces(nullptr)) return;
+      if (!forces(nullptr, nullptr)) return;
       if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
     }
+    const size_t record = (size_t)(rec.k0 + s + 1u) * v.n_slots;
+    if (kVerlet && s > 0u && (kObs || rec.lam)) epilogue(s - 1u, ke_other);
     uint32_t scaled = 0xffffffffu;
     float lam = 1.0f;
     for (uint32_t b = b0; b < b1; ++b) {
@@ -363,15 +386,21 @@ k_run(DeviceView v, RunView rv, uint32_t n_steps, float sd_dmax, float sd_fref) 
       }
       scaled = r;
       pre_block<kPre>(v, p, &v.rs[r], b, p.check_every == 1u ? 0ull : v.rs[r].step + s + 1ull, lam,
-                      sd_dmax, sd_fref, &rv.ctl->any[s & 1u]);
+                      sd_dmax, sd_fref, &rv.ctl->any[s & 1u],
+                      kVerlet && rec.pos ? rec.pos + record : nullptr);
       if (kVerlet && p.skin == 0.0f && threadIdx.x == 0) rv.ctl->any[s & 1u] = 1u;
     }
     if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
     if (__ldcg(&rv.ctl->any[s & 1u]) != 0u) {  // launch-uniform
-      if (blockIdx.x == 0) run_decide<kPre>(v, rv, since, s);
+      if (blockIdx.x == 0) run_decide<kPre>(v, rv, rec, since, s);
       since = s + 1u;
       if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
       if (!run_rebuild(v, rv, sh, target)) return;
+      if (kVerlet && rec.snap_nbr && v.work_start[v.n_replicas] != 0u) {
+        for_listed_blocks(v, [&](uint32_t b) {
+          snapshot_block(v, b, rec.snap_nbr + record * v.nbr_stride, rec.snap_cnt + record);
+        });
+      }
     }
     // What follows is not read before the next barrier.
     if (gthread == 0u) rv.ctl->any[(s + 1u) & 1u] = 0u;
@@ -382,17 +411,19 @@ k_run(DeviceView v, RunView rv, uint32_t n_steps, float sd_dmax, float sd_fref) 
           z[k] = make_longlong2(0, 0);
         }
       }
-      if (!forces(ke)) return;
+      if (!forces(ke, rec.vel ? rec.vel + record : nullptr)) return;
       if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
     }
   }
   if (kVerlet) {
     long long* ke = (n_steps & 1u) ? v.ke_part : rv.ke_odd;  // of the last step
+    if (kObs || rec.lam) epilogue(n_steps - 1u, ke);
     for (uint32_t r = blockIdx.x * kBuildWarps + warp; r < v.n_replicas;
          r += gridDim.x * kBuildWarps) {
       double kin = 0.0;
       if (kinetic) {
         kin = bucket_kinetic(ke, r, lane);
+        __syncwarp();
         longlong2* z = reinterpret_cast<longlong2*>(ke) + (size_t)r * kKeBuckets;
         for (uint32_t k = lane; k < kKeBuckets; k += 32u) z[k] = make_longlong2(0, 0);
       }
@@ -403,7 +434,9 @@ k_run(DeviceView v, RunView rv, uint32_t n_steps, float sd_dmax, float sd_fref) 
           st->need_rebuild = 0u;
           st->reorder_now = 0u;
         }
-        finish_replica<kObs>(v, r, true, kinetic, n_steps, kin);
+        st->lambda = kinetic ? berendsen_lambda(v.rp[r], kin) : 1.0;
+        st->step += n_steps;
+        if (kinetic) st->last_kinetic = kin;
       }
     }
   }
@@ -425,7 +458,7 @@ void check(cudaError_t e) {
 }
 
 template <int kPre, bool kObs, int kTpa, int kNt>
-void launch_one(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
+void launch_one(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uint32_t n_steps) {
   auto* kernel = k_run<kPre, kObs, kTpa, kNt>;
   // One wave at most.  Pair-force items of a small system leave blocks idle,
   // but a rebuild shares its cells over every warp, and barriers take the same
@@ -449,27 +482,28 @@ void launch_one(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  check(cudaLaunchKernelEx(&cfg, kernel, l.v, rv, n_steps, l.sd_dmax, l.sd_fref));
+  check(cudaLaunchKernelEx(&cfg, kernel, l.v, rv, rec, n_steps, l.sd_dmax, l.sd_fref));
 }
 
 }  // namespace
 
 // Four threads per particle: a small system has threads to spare, and its
 // steps take as long as a thread's list.
-void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables) {
+void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables,
+                const RunRecord& rec) {
   if (observables) {
-    launch_one<kPreVerlet, true, 4, 0>(l, rv, n_steps);
+    launch_one<kPreVerlet, true, 4, 0>(l, rv, rec, n_steps);
   } else if (l.lj_types == 1) {
-    launch_one<kPreVerlet, false, 4, 1>(l, rv, n_steps);
+    launch_one<kPreVerlet, false, 4, 1>(l, rv, rec, n_steps);
   } else if (l.lj_types == 2) {
-    launch_one<kPreVerlet, false, 4, 2>(l, rv, n_steps);
+    launch_one<kPreVerlet, false, 4, 2>(l, rv, rec, n_steps);
   } else {
-    launch_one<kPreVerlet, false, 4, 0>(l, rv, n_steps);
+    launch_one<kPreVerlet, false, 4, 0>(l, rv, rec, n_steps);
   }
 }
 
 void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
-  launch_one<kPreDescent, false, 4, 0>(l, rv, n_steps);
+  launch_one<kPreDescent, false, 4, 0>(l, rv, RunRecord{}, n_steps);
 }
 
 uint32_t run_scan_chunks(uint32_t total_cells) {

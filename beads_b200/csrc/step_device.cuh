@@ -27,7 +27,7 @@ template <int kMode>
 __device__ __forceinline__ void pre_block(const DeviceView& v, const ReplicaParams& p,
                                           ReplicaState* st, uint32_t b, unsigned long long phys,
                                           float lam, float sd_dmax, float sd_fref,
-                                          unsigned* any) {
+                                          unsigned* any, float4* record) {
   const uint32_t slot = b * kBlock + threadIdx.x;
   const uint32_t local = slot - p.atom_begin;
   const bool check_step = is_check_step<kMode>(p, phys);
@@ -65,6 +65,7 @@ __device__ __forceinline__ void pre_block(const DeviceView& v, const ReplicaPara
     x.y = __fmaf_rn(-cy, p.len[1], x.y);
     x.z = __fmaf_rn(-cz, p.len[2], x.z);
     v.pos[slot] = x;
+    if (record) record[slot] = x;
     // Images and the crossing count change only on a boundary crossing, so
     // a step reads neither image vector otherwise.
     uint32_t cross = 0u;
@@ -922,7 +923,7 @@ enum ForceMode : int {
 __device__ __forceinline__ double post_slot_vm(const DeviceView& v, const ReplicaParams& p,
                                                ReplicaState* st, uint32_t i, bool real, bool kick,
                                                bool kinetic, float4 vm, float fx, float fy,
-                                               float fz) {
+                                               float fz, float4* record = nullptr) {
   double ke = 0.0;
   if (real) {
     if (kick) {
@@ -931,6 +932,7 @@ __device__ __forceinline__ double post_slot_vm(const DeviceView& v, const Replic
       vm.y = __fmaf_rn(h, fy, vm.y);
       vm.z = __fmaf_rn(h, fz, vm.z);
       v.vel[i] = vm;
+      if (record) record[i] = vm;
       if (!isfinite(vm.x + vm.y + vm.z)) atomicOr(&st->status, kStatusNonFinite);
     }
     if (kinetic) {
@@ -943,9 +945,10 @@ __device__ __forceinline__ double post_slot_vm(const DeviceView& v, const Replic
 
 __device__ __forceinline__ double post_slot(const DeviceView& v, const ReplicaParams& p,
                                             ReplicaState* st, uint32_t i, bool real, bool kick,
-                                            bool kinetic, float fx, float fy, float fz) {
+                                            bool kinetic, float fx, float fy, float fz,
+                                            float4* record = nullptr) {
   const float4 vm = real ? v.vel[i] : make_float4(0.f, 0.f, 0.f, 1.f);
-  return post_slot_vm(v, p, st, i, real, kick, kinetic, vm, fx, fy, fz);
+  return post_slot_vm(v, p, st, i, real, kick, kinetic, vm, fx, fy, fz, record);
 }
 
 // Berendsen scale of the velocities after a step of kinetic energy `kin`
@@ -957,34 +960,57 @@ __device__ __forceinline__ double berendsen_lambda(const ReplicaParams& p, doubl
   return sqrt(arg > 0.0 ? arg : 0.0);
 }
 
-// Per-replica epilogue of `steps` steps whose last left the kinetic energy
-// kin (one thread): pending scale, step counter, observables.
+// Observables of a step of replica r that left the kinetic energy kin and the
+// scale lam (one thread); takes and clears the step's totals.
+__device__ __forceinline__ ReplicaObs take_observables(ReplicaState* st, unsigned long long step,
+                                                       double kin, double lam) {
+  ReplicaObs o;
+  o.step = step;
+  o.pair_pe = take_total(st, kAccPair);
+  o.bond_pe = take_total(st, kAccBond);
+  o.angle_pe = take_total(st, kAccAngle);
+  o.dihedral_pe = take_total(st, kAccDihedral);
+  o.virial = take_total(st, kAccVirial);
+  o.ke_pre = kin;
+  o.lambda = lam;
+  o.builds = st->builds;
+  o.dangerous = st->dangerous;
+  o.status = st->status;
+  o.pad = 0;
+  return o;
+}
+
+// Per-replica epilogue of a step that left the kinetic energy kin (one
+// thread): pending scale, step counter, observables.
 template <bool kObs>
 __device__ __forceinline__ void finish_replica(const DeviceView& v, uint32_t r, bool kick,
-                                               bool kinetic, unsigned long long steps,
-                                               double kin) {
+                                               bool kinetic, double kin) {
   ReplicaState* st = &v.rs[r];
   const double lam = kick && kinetic ? berendsen_lambda(v.rp[r], kin) : 1.0;
   if (kick) {
     st->lambda = lam;
-    st->step += steps;
+    st->step += 1ull;
   }
   if (kinetic) st->last_kinetic = kin;
-  if (kObs) {
-    ReplicaObs o;
-    o.step = st->step;
-    o.pair_pe = take_total(st, kAccPair);
-    o.bond_pe = take_total(st, kAccBond);
-    o.angle_pe = take_total(st, kAccAngle);
-    o.dihedral_pe = take_total(st, kAccDihedral);
-    o.virial = take_total(st, kAccVirial);
-    o.ke_pre = kin;
-    o.lambda = lam;
-    o.builds = st->builds;
-    o.dangerous = st->dangerous;
-    o.status = st->status;
-    o.pad = 0;
-    v.obs[r] = o;
+  if (kObs) v.obs[r] = take_observables(st, st->step, kin, lam);
+}
+
+// Copies the list rows (and counts) of 128-slot block b into a snapshot of the
+// list.  A block's rows are whole interleave groups, whose entries up to the
+// longest row are contiguous (the rest of a group is never read).
+__device__ __forceinline__ void snapshot_block(const DeviceView& v, uint32_t b, uint32_t* nbr,
+                                               uint32_t* cnt) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  constexpr uint32_t kGroups = kBlock / kGroup;
+  for (uint32_t g = warp; g < kGroups; g += blockDim.x >> 5) {
+    const uint32_t row = b * kBlock + g * kGroup;
+    const uint32_t n = lane < (uint32_t)kGroup ? v.nbr_count[row + lane] : 0u;
+    if (lane < (uint32_t)kGroup) cnt[row + lane] = n;
+    const uint64_t at = nbr_index(row, 0, v.nbr_stride);
+    const uint32_t words = __reduce_max_sync(kFull, n) * kGroup;
+    const uint4* src = reinterpret_cast<const uint4*>(v.nbr + at);
+    uint4* dst = reinterpret_cast<uint4*>(nbr + at);
+    for (uint32_t t = lane; t < words / 4u; t += 32u) dst[t] = __ldcs(src + t);
   }
 }
 
@@ -1261,7 +1287,8 @@ __device__ __forceinline__ void lj_pairs(const DeviceView& v, const ReplicaParam
 template <bool kObs, bool kClamp, int kTpa, int kUnroll, bool kNoL1, int kNt, bool kCoh>
 __device__ __forceinline__ void lj_block(const DeviceView& v, const ReplicaParams& p, uint32_t r,
                                          uint32_t item, const LjCoeff* table, bool post,
-                                         bool kinetic, long long* ke_part) {
+                                         bool kinetic, long long* ke_part,
+                                         float4* record = nullptr) {
   constexpr uint32_t kAtoms = kBlock / kTpa;  // particles per block
   const uint32_t sb = item / kTpa;            // 128-slot block of the particles
   const int nt = p.n_types;
@@ -1313,7 +1340,7 @@ __device__ __forceinline__ void lj_block(const DeviceView& v, const ReplicaParam
   if (sub == 0u) v.force[i] = make_float4(fx, fy, fz, 0.f);
   ReplicaState* st = &v.rs[r];
   double ke = 0.0;
-  if (post) ke = post_slot_vm(v, p, st, i, owner, true, kinetic, vm_kick, fx, fy, fz);
+  if (post) ke = post_slot_vm(v, p, st, i, owner, true, kinetic, vm_kick, fx, fy, fz, record);
   if (kObs) {
     const float e = ae.total(), w = -aw.total();
     block_add_lane<kBlock>(owner, 0.5 * (double)e, st, kAccPair);
@@ -1541,7 +1568,7 @@ __device__ __forceinline__ void bonded_term(const DeviceView& v, uint32_t t) {
 template <bool kObs>
 __device__ __forceinline__ void bonded_block(const DeviceView& v, const ReplicaParams& p,
                                              uint32_t r, uint32_t b, bool post, bool kinetic,
-                                             long long* ke_part) {
+                                             long long* ke_part, float4* record = nullptr) {
   const uint32_t i = b * kBlock + threadIdx.x;
   const bool real = (i - p.atom_begin) < p.n_atoms;
   float eb = 0.f, ea = 0.f, ed = 0.f, w = 0.f;
@@ -1579,7 +1606,7 @@ __device__ __forceinline__ void bonded_block(const DeviceView& v, const ReplicaP
   }
   ReplicaState* st = &v.rs[r];
   double ke = 0.0;
-  if (post) ke = post_slot(v, p, st, i, real, true, kinetic, fo.x, fo.y, fo.z);
+  if (post) ke = post_slot(v, p, st, i, real, true, kinetic, fo.x, fo.y, fo.z, record);
   if (kObs) {
     block_add_lane<kBlock>(real, eb, st, kAccBond);
     block_add_lane<kBlock>(real, ea, st, kAccAngle);

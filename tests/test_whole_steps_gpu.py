@@ -121,3 +121,33 @@ def test_descent_cut_into_launches(iterations):
         # every call builds its lists anew: the same sets, summed in the same order
         assert np.abs(outs[0]["positions"] - outs[1]["positions"]).max() < 1e-3
     assert np.isfinite(outs[0]["positions"]).all()
+
+
+@pytest.mark.parametrize("checkpoint", [0, 7, 80])
+def test_recorded_steps_give_the_gradients_of_separate_launches(checkpoint):
+    """The forward window (more steps than one launch keeps observables of) and
+    the replayed segments recorded by the step kernel, against recordings made
+    between separate launches."""
+    import torch
+
+    from beads_b200.adjoint import trajectory_observables
+
+    specs = workloads.fit_mixture(n_replicas=2, n=700, seed=3) + [
+        dataclasses.replace(workloads.fit_mixture(n_replicas=1, n=700, seed=9)[0], thermostat=None)]
+    outs = []
+    for whole in (True, False):
+        with Engine(specs) as eng:
+            if not whole:
+                eng.set_tuning(2, False, 4, True)
+            leaves = [torch.tensor(specs[0].epsilon).requires_grad_(True),
+                      torch.tensor(specs[0].sigma).requires_grad_(True),
+                      torch.tensor(np.concatenate([s.positions for s in specs])).requires_grad_(True),
+                      torch.tensor(np.concatenate([s.velocities for s in specs])).requires_grad_(True)]
+            obs = trajectory_observables(eng, *leaves, steps=80, record_from=10,
+                                         checkpoint_every=checkpoint)
+            grads = torch.autograd.grad((obs * torch.linspace(0.5, 1.5, obs.numel(),
+                                                              dtype=obs.dtype).view_as(obs)).sum(),
+                                        leaves)
+            outs.append([obs.detach(), *grads])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
