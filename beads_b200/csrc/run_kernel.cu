@@ -92,12 +92,19 @@ __device__ __forceinline__ void for_listed_blocks(const DeviceView& v, F&& f) {
 }
 
 constexpr uint32_t kMinGrid = 296;
+// Threads per particle of the pair forces: a small system has threads to
+// spare, and its steps take as long as a thread's share of a list.
+constexpr int kRunTpa = 4;
+// Contexts whose pair forces fit two blocks per SM in one pass keep eight list
+// entries in flight per thread instead of four, at the registers of four
+// blocks per SM.
+constexpr int kSmallBlocksPerSm = 4;
+constexpr uint32_t kSmallItems = 2u * 148u;
 constexpr uint32_t kRunScanPer = 4;                        // consecutive cells per thread
 constexpr uint32_t kRunScanChunk = kBlock * kRunScanPer;  // work items per block of the scan
+// Replicas of up to this many cells are scanned by one block each.
+constexpr uint32_t kRunScanCells = 4u * kRunScanChunk;
 
-// Rebuild decision of every replica and the work lists of the rebuilding ones
-// (block 0): work_start / chain_block_start / work_atoms hold the cells, slot
-// blocks and particles of the rebuilding replicas before each replica.
 // Steps since + 1 .. step - 1 of the launch moved no slot far enough; their
 // checks are counted here.
 __device__ __forceinline__ void count_checks(const ReplicaParams& p, ReplicaState* st,
@@ -109,62 +116,12 @@ __device__ __forceinline__ void count_checks(const ReplicaParams& p, ReplicaStat
                                 : (uint32_t)(hi / p.check_every - lo / p.check_every);
 }
 
-template <int kPre>
-__device__ void run_decide(const DeviceView& v, const RunView& rv, const RunRecord& rec,
-                           uint32_t since, uint32_t step) {
-  uint32_t cells = 0, blocks = 0, atoms = 0, reorder = 0;
-  for (uint32_t base = 0; base < v.n_replicas; base += kBlock) {
-    const uint32_t r = base + threadIdx.x;
-    uint32_t c = 0, b = 0, n = 0;
-    bool move = false;
-    if (r < v.n_replicas) {
-      ReplicaState* st = &v.rs[r];
-      if (kPre == kPreVerlet) count_checks(v.rp[r], st, since, step);
-      if (decide_replica<kPre>(v.rp[r], st, st->step + step + 1ull)) {
-        c = v.rp[r].n_cells;
-        b = v.rp[r].n_pad / kBlock;
-        n = v.rp[r].n_atoms;
-        move = st->reorder_now != 0u;
-        if (rec.flags) rec.flags[(size_t)(rec.k0 + step + 1u) * v.n_replicas + r] = 1u;
-      }
-    }
-    uint32_t tc, tb, tn;
-    const uint32_t ec = block_exclusive_scan<kBlock>(c, tc);
-    const uint32_t eb = block_exclusive_scan<kBlock>(b, tb);
-    const uint32_t en = block_exclusive_scan<kBlock>(n, tn);
-    if (r < v.n_replicas) {
-      v.work_start[r] = cells + ec;
-      v.chain_block_start[r] = blocks + eb;
-      rv.work_atoms[r] = atoms + en;
-    }
-    cells += tc;
-    blocks += tb;
-    atoms += tn;
-    reorder |= __syncthreads_or(move ? 1 : 0);
-  }
-  if (threadIdx.x == 0) {
-    v.work_start[v.n_replicas] = cells;
-    v.chain_block_start[v.n_replicas] = blocks;
-    rv.work_atoms[v.n_replicas] = atoms;
-    rv.ctl->reorder = reorder;
-    if (cells != 0u) *v.chain_launches += 1ull;
-  }
-}
-
-// The rebuild chain of the replicas run_decide listed; false after a barrier
-// that ran out.
-__device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& rv,
-                                            RunShared& sh, uint32_t& target) {
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t items = v.work_start[v.n_replicas];
-  if (items == 0u) return true;  // launch-uniform
-  const bool reorder = rv.ctl->reorder != 0u;
-  for_listed_blocks(v, [&](uint32_t b) { bin_block(v, b); });
-  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
-  // Cell starts: totals of kRunScanChunk consecutive work items, then each
-  // chunk adds the totals before it.  Every particle of a rebuilding replica
-  // is counted once, so the running total of a replica's first cell is
-  // work_atoms.
+// Cell starts of large replicas, the work items in chunks of kRunScanChunk:
+// chunk totals, then each chunk adds the totals before it.  Every particle of
+// a rebuilding replica is counted once, so the running total of a replica's
+// first cell is work_atoms.  False after a barrier that ran out.
+__device__ __forceinline__ bool run_scan(const DeviceView& v, const RunView& rv, uint32_t items,
+                                         uint32_t& target) {
   const uint32_t chunks = (items + kRunScanChunk - 1u) / kRunScanChunk;
   for (uint32_t ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
     uint32_t s = 0;
@@ -214,8 +171,126 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
       run += cnt[k];
     }
   }
+  return grid_barrier(rv.ctl, &v.rs->status, target);
+}
+
+// The work lists of the replicas that rebuild in this step (the last block):
+// work_start / chain_block_start / work_atoms hold the cells, slot blocks and
+// particles of the rebuilding replicas before each replica.  The replicas'
+// state is left alone: other blocks read it meanwhile.
+template <int kPre>
+__device__ void run_plan(const DeviceView& v, const RunView& rv, const RunRecord& rec,
+                         uint32_t step) {
+  uint32_t cells = 0, blocks = 0, atoms = 0;
+  bool reorder = false, wide = false;
+  for (uint32_t base = 0; base < v.n_replicas; base += kBlock) {
+    const uint32_t r = base + threadIdx.x;
+    uint32_t c = 0, b = 0, n = 0;
+    if (r < v.n_replicas) {
+      const ReplicaParams& p = v.rp[r];
+      const ReplicaState* st = &v.rs[r];
+      if (needs_rebuild<kPre>(p, st, st->step + step + 1ull)) {
+        c = p.n_cells;
+        b = p.n_pad / kBlock;
+        n = p.n_atoms;
+        reorder |= p.sort_every > 0u && (st->builds + 1ull) % p.sort_every == 0ull;
+        wide |= c > kRunScanCells;
+        if (rec.flags) rec.flags[(size_t)(rec.k0 + step + 1u) * v.n_replicas + r] = 1u;
+      }
+    }
+    uint32_t tc = c, tb = b, tn = n, ec = 0, eb = 0, en = 0;
+    if (v.n_replicas > 1u) {
+      ec = block_exclusive_scan<kBlock>(c, tc);
+      eb = block_exclusive_scan<kBlock>(b, tb);
+      en = block_exclusive_scan<kBlock>(n, tn);
+    }
+    if (r < v.n_replicas) {
+      v.work_start[r] = cells + ec;
+      v.chain_block_start[r] = blocks + eb;
+      rv.work_atoms[r] = atoms + en;
+    }
+    cells += tc;
+    blocks += tb;
+    atoms += tn;
+  }
+  reorder = __syncthreads_or(reorder);
+  wide = __syncthreads_or(wide);
+  if (threadIdx.x == 0) {
+    v.work_start[v.n_replicas] = cells;
+    v.chain_block_start[v.n_replicas] = blocks;
+    rv.work_atoms[v.n_replicas] = atoms;
+    rv.ctl->reorder = reorder ? 1u : 0u;
+    rv.ctl->wide = wide ? 1u : 0u;
+    if (cells != 0u) *v.chain_launches += 1ull;
+  }
+}
+
+// The rebuild chain after a drift in which some slot moved half the skin;
+// blocks bin, scatter and reorder the slot blocks [b0, b1) they drift.  False
+// after a barrier that ran out.  A barrier and the loads behind it cost 2-3 us,
+// so the stages are few: the plan is made while the slots are binned, and the
+// replicas' state advances while the cells are scanned.
+template <int kPre>
+__device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& rv,
+                                            const RunRecord& rec, RunShared& sh, uint32_t b0,
+                                            uint32_t b1, uint32_t since, uint32_t step,
+                                            uint32_t& target) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  if (blockIdx.x == gridDim.x - 1u) run_plan<kPre>(v, rv, rec, step);
+  for (uint32_t b = b0; b < b1; ++b) {
+    const uint32_t r = v.block_replica[b];
+    const ReplicaState* st = &v.rs[r];
+    if (needs_rebuild<kPre>(v.rp[r], st, st->step + step + 1ull)) bin_slots(v, v.rp[r], b);
+  }
   if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
-  for_listed_blocks(v, [&](uint32_t b) { scatter_block(v, b); });
+  const uint32_t items = v.work_start[v.n_replicas];
+  const bool reorder = rv.ctl->reorder != 0u;
+  const bool wide = rv.ctl->wide != 0u;
+  for (uint32_t r = (gridDim.x - 1u - blockIdx.x) * kBlock + threadIdx.x; r < v.n_replicas;
+       r += gridDim.x * kBlock) {
+    ReplicaState* st = &v.rs[r];
+    if (kPre == kPreVerlet) count_checks(v.rp[r], st, since, step);
+    decide_replica<kPre>(v.rp[r], st, st->step + step + 1ull);
+  }
+  if (items == 0u) return grid_barrier(rv.ctl, &v.rs->status, target);  // launch-uniform
+  if (!wide) {
+    // Cell starts, a block per rebuilding replica.
+    for (uint32_t r = blockIdx.x; r < v.n_replicas; r += gridDim.x) {
+      if (v.work_start[r] == v.work_start[r + 1u]) continue;  // block-uniform
+      const ReplicaParams& p = v.rp[r];
+      uint32_t* count = v.cell_count + p.cell_begin;
+      uint32_t* start = v.cell_start + p.start_base;
+      uint32_t* cursor = v.cell_cursor + p.cell_begin;
+      uint32_t run = p.atom_begin;
+      const uint32_t n_cells = p.n_cells;
+      for (uint32_t base = 0; base < n_cells; base += kRunScanChunk) {
+        const uint32_t c0 = base + threadIdx.x * kRunScanPer;
+        uint32_t cnt[kRunScanPer], s = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kRunScanPer; ++k) {
+          cnt[k] = c0 + k < n_cells ? __ldcg(&count[c0 + k]) : 0u;
+          s += cnt[k];
+        }
+        uint32_t total;
+        uint32_t at = run + block_exclusive_scan<kBlock>(s, total);
+#pragma unroll
+        for (uint32_t k = 0; k < kRunScanPer; ++k) {
+          if (c0 + k < n_cells) {
+            start[c0 + k] = at;
+            cursor[c0 + k] = at;
+            count[c0 + k] = 0u;
+          }
+          at += cnt[k];
+        }
+        run += total;
+      }
+      if (threadIdx.x == 0) start[n_cells] = run;
+    }
+    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  } else if (!run_scan(v, rv, items, target)) {
+    return false;
+  }
+  for (uint32_t b = b0; b < b1; ++b) scatter_block(v, b);
   if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
   if (rv.any_sparse) {
     for (uint32_t w = blockIdx.x * kBlock + threadIdx.x; w < items; w += gridDim.x * kBlock) {
@@ -229,12 +304,12 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
   }
   if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
   if (reorder) {
-    for_listed_blocks(v, [&](uint32_t b) { reorder_gather_block(v, b); });
+    for (uint32_t b = b0; b < b1; ++b) reorder_gather_block(v, b);
     if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
-    for_listed_blocks(v, [&](uint32_t b) { reorder_commit_block(v, b); });
+    for (uint32_t b = b0; b < b1; ++b) reorder_commit_block(v, b);
     if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
     if (v.excl_cap > 0u) {
-      for_listed_blocks(v, [&](uint32_t b) { project_exclusions_block(v, b, false); });
+      for (uint32_t b = b0; b < b1; ++b) project_exclusions_block(v, b, false);
       if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
     }
   }
@@ -276,8 +351,8 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
 // kPre: velocity Verlet (drift, rebuild, forces and second half-kick per step)
 // or the capped descent (forces, move, rebuild per iteration).  kObs: energies
 // and virial of every step.
-template <int kPre, bool kObs, int kTpa, int kNt>
-__global__ void __launch_bounds__(kBlock, kRunBlocksPerSm)
+template <int kPre, bool kObs, int kNt, bool kSmall>
+__global__ void __launch_bounds__(kBlock, kSmall ? kSmallBlocksPerSm : kRunBlocksPerSm)
 k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, float sd_fref) {
   constexpr bool kVerlet = kPre == kPreVerlet;
   __shared__ RunShared sh;
@@ -295,7 +370,7 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
   // neighbours are mostly those of the item before it.
   const uint32_t b0 = (uint32_t)((uint64_t)v.n_blocks * blockIdx.x / gridDim.x);
   const uint32_t b1 = (uint32_t)((uint64_t)v.n_blocks * (blockIdx.x + 1u) / gridDim.x);
-  const uint32_t n_items = v.n_blocks * kTpa;
+  const uint32_t n_items = v.n_blocks * kRunTpa;
   const uint32_t i0 = (uint32_t)((uint64_t)n_items * blockIdx.x / gridDim.x);
   const uint32_t i1 = (uint32_t)((uint64_t)n_items * (blockIdx.x + 1u) / gridDim.x);
 
@@ -319,8 +394,8 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
 
   auto forces = [&](long long* ke, float4* vel) -> bool {
     for (uint32_t item = i0; item < i1; ++item) {
-      enter(replica_of(item / kTpa));
-      lj_block<kObs, !kVerlet, kTpa, 4, true, kNt, true>(v, p, cur, item, table,
+      enter(replica_of(item / kRunTpa));
+      lj_block<kObs, !kVerlet, kRunTpa, kSmall ? 8 : 4, true, kNt, true>(v, p, cur, item, table,
                                                          kVerlet && !bonded, kinetic, ke, vel);
     }
     if (bonded) {
@@ -392,10 +467,8 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
     }
     if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
     if (__ldcg(&rv.ctl->any[s & 1u]) != 0u) {  // launch-uniform
-      if (blockIdx.x == 0) run_decide<kPre>(v, rv, rec, since, s);
+      if (!run_rebuild<kPre>(v, rv, rec, sh, b0, b1, since, s, target)) return;
       since = s + 1u;
-      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
-      if (!run_rebuild(v, rv, sh, target)) return;
       if (kVerlet && rec.snap_nbr && v.work_start[v.n_replicas] != 0u) {
         for_listed_blocks(v, [&](uint32_t b) {
           snapshot_block(v, b, rec.snap_nbr + record * v.nbr_stride, rec.snap_cnt + record);
@@ -457,9 +530,9 @@ void check(cudaError_t e) {
   }
 }
 
-template <int kPre, bool kObs, int kTpa, int kNt>
-void launch_one(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uint32_t n_steps) {
-  auto* kernel = k_run<kPre, kObs, kTpa, kNt>;
+template <int kPre, bool kObs, int kNt, bool kSmall>
+void launch_as(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uint32_t n_steps) {
+  auto* kernel = k_run<kPre, kObs, kNt, kSmall>;
   // One wave at most.  Pair-force items of a small system leave blocks idle,
   // but a rebuild shares its cells over every warp, and barriers take the same
   // time up to about two blocks per SM.
@@ -474,7 +547,7 @@ void launch_one(const StepLaunch& l, const RunView& rv, const RunRecord& rec, ui
     return (uint32_t)(sms * per_sm);
   }();
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(std::min(wave, std::max(kMinGrid, l.v.n_blocks * (uint32_t)kTpa)));
+  cfg.gridDim = dim3(std::min(wave, std::max(kMinGrid, l.v.n_blocks * (uint32_t)kRunTpa)));
   cfg.blockDim = dim3(kBlock);
   cfg.stream = l.stream;
   cudaLaunchAttribute attr[1];
@@ -485,25 +558,32 @@ void launch_one(const StepLaunch& l, const RunView& rv, const RunRecord& rec, ui
   check(cudaLaunchKernelEx(&cfg, kernel, l.v, rv, rec, n_steps, l.sd_dmax, l.sd_fref));
 }
 
+template <int kPre, bool kObs, int kNt>
+void launch_one(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uint32_t n_steps) {
+  if (l.v.n_blocks * (uint32_t)kRunTpa <= kSmallItems) {
+    launch_as<kPre, kObs, kNt, true>(l, rv, rec, n_steps);
+  } else {
+    launch_as<kPre, kObs, kNt, false>(l, rv, rec, n_steps);
+  }
+}
+
 }  // namespace
 
-// Four threads per particle: a small system has threads to spare, and its
-// steps take as long as a thread's list.
 void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables,
                 const RunRecord& rec) {
   if (observables) {
-    launch_one<kPreVerlet, true, 4, 0>(l, rv, rec, n_steps);
+    launch_one<kPreVerlet, true, 0>(l, rv, rec, n_steps);
   } else if (l.lj_types == 1) {
-    launch_one<kPreVerlet, false, 4, 1>(l, rv, rec, n_steps);
+    launch_one<kPreVerlet, false, 1>(l, rv, rec, n_steps);
   } else if (l.lj_types == 2) {
-    launch_one<kPreVerlet, false, 4, 2>(l, rv, rec, n_steps);
+    launch_one<kPreVerlet, false, 2>(l, rv, rec, n_steps);
   } else {
-    launch_one<kPreVerlet, false, 4, 0>(l, rv, rec, n_steps);
+    launch_one<kPreVerlet, false, 0>(l, rv, rec, n_steps);
   }
 }
 
 void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
-  launch_one<kPreDescent, false, 4, 0>(l, rv, RunRecord{}, n_steps);
+  launch_one<kPreDescent, false, 0>(l, rv, RunRecord{}, n_steps);
 }
 
 uint32_t run_scan_chunks(uint32_t total_cells) {

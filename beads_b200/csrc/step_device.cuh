@@ -96,6 +96,16 @@ __device__ __forceinline__ void pre_block(const DeviceView& v, const ReplicaPara
   }
 }
 
+// Whether a replica rebuilds its list in step `phys`, as decide_replica will
+// decide it (no state is changed).
+template <int kMode>
+__device__ __forceinline__ bool needs_rebuild(const ReplicaParams& p, const ReplicaState* st,
+                                              unsigned long long phys) {
+  if (st->status & (kStatusNonFinite | kStatusFixedOverflow)) return false;
+  if (kMode == kPreVerlet && p.skin == 0.0f) return true;
+  return st->exceeded != 0u && is_check_step<kMode>(p, phys);
+}
+
 // The rebuild decision of one replica for step `phys` (neighbor_system.cpp:79-105).
 template <int kMode>
 __device__ __forceinline__ unsigned decide_replica(const ReplicaParams& p, ReplicaState* st,
@@ -164,10 +174,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t& t
 }
 
 // rebuild 1: cell id and per-cell count.
-__device__ __forceinline__ void bin_block(const DeviceView& v, uint32_t b) {
-  const uint32_t r = v.block_replica[b];
-  if (!v.rs[r].need_rebuild) return;
-  const ReplicaParams& p = v.rp[r];
+__device__ __forceinline__ void bin_slots(const DeviceView& v, const ReplicaParams& p, uint32_t b) {
   const uint32_t slot = b * kBlock + threadIdx.x;
   const uint32_t local = slot - p.atom_begin;
   if (local >= p.n_atoms) return;
@@ -178,6 +185,11 @@ __device__ __forceinline__ void bin_block(const DeviceView& v, uint32_t b) {
   const uint32_t cell = p.cell_begin + ix + p.nc[0] * (iy + p.nc[1] * iz);
   v.cell_of_slot[slot] = cell;
   atomicAdd(&v.cell_count[cell], 1u);
+}
+
+__device__ __forceinline__ void bin_block(const DeviceView& v, uint32_t b) {
+  const uint32_t r = v.block_replica[b];
+  if (v.rs[r].need_rebuild) bin_slots(v, v.rp[r], b);
 }
 
 // rebuild 3: scatter slots into their cells (order inside a cell is fixed by
