@@ -294,19 +294,21 @@ k_project_exclusions(DeviceView v, int force_all) {
   project_exclusions_block(v, blockIdx.x, force_all != 0);
 }
 
-// Warp w builds the lists of work item w (k_scan): the warps past the cells
-// of the rebuilding replicas return after one load.
+// Warps w parts .. w parts + parts - 1 build the lists of work item w (k_scan),
+// a share of its cell's particles each: the warps past the cells of the
+// rebuilding replicas return after one load.
 template <bool kExcl, bool kByQ>
-__global__ void __launch_bounds__(kBlock, 7) k_build(DeviceView v) {
+__global__ void __launch_bounds__(kBlock, 7) k_build(DeviceView v, uint32_t parts) {
   __shared__ BuildShared sh[kBuildWarps];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t w = blockIdx.x * kBuildWarps + warp;
+  const uint32_t k = blockIdx.x * kBuildWarps + warp;
+  const uint32_t w = k / parts;
   if (w >= v.work_start[v.n_replicas]) return;  // warp-uniform
   const uint32_t r = work_replica(v, w);
   const ReplicaParams& p = v.rp[r];
   if (p.sparse) return;  // built by k_build_sparse
   build_cell<kExcl, kByQ>(v, p, &v.rs[r], p.cell_begin + (w - v.work_start[r]), lane, sh[warp],
-                           0u, 1u);
+                           k - w * parts, parts);
 }
 
 template <bool kExcl, bool kByQ>
@@ -731,10 +733,17 @@ void launch_rebuild(const StepLaunch& l, bool force_all, bool count_build) {
     k_project_exclusions<<<l.v.n_blocks, kBlock, 0, l.stream>>>(l.v, 0);
     check_launch("project_exclusions");
   }
-  const uint32_t bg = (l.v.total_cells + kBuildWarps - 1) / kBuildWarps;
+  // Shares of a cell per warp.  A warp takes ~100 us for a cell of 20
+  // particles, so cells that do not fill several waves of warps (4,144) leave
+  // the last wave nearly empty: in a batch only the rebuilding replicas' cells
+  // count, a fraction of the grid.  Measured with 1 / 2 / 3 / 4 shares: 128
+  // replicas (832,000 beads) 491 / 412 / 400 / 402 us a step, 100,003 beads
+  // 46.9 / 46.6 / 47.1 / 47.2, 1,048,576 beads 238 / 240 / 245 / 250.
+  const uint32_t parts = l.v.n_replicas > 1u ? 3u : l.v.total_cells < 16384u ? 2u : 1u;
+  const uint32_t bg = (l.v.total_cells * parts + kBuildWarps - 1) / kBuildWarps;
 #define BB_BUILD(excl, q)                                                                  \
   do {                                                                                     \
-    if (l.any_dense) k_build<excl, q><<<bg, kBlock, 0, l.stream>>>(l.v);                   \
+    if (l.any_dense) k_build<excl, q><<<bg, kBlock, 0, l.stream>>>(l.v, parts);                   \
     if (l.any_sparse) k_build_sparse<excl, q><<<l.v.n_blocks, kBlock, 0, l.stream>>>(l.v); \
   } while (0)
   if (l.excl_cap > 0) {
