@@ -850,6 +850,7 @@ void Engine::adjoint_forward(uint64_t steps, uint64_t record_from, uint32_t ever
                    "memset");
       }
       rec.obs = A.obs_ring;
+      obs_downloaded_ = false;
       launch_run(launch_, run_, static_cast<uint32_t>(m), observe, rec);
       step_ += m;
       if (observe) {

@@ -137,11 +137,33 @@ void Engine::tuning(int* tpa, int* fuse_post, int* unroll, int* no_l1, int* auto
 // launches and the conditional node (~20 us of a step) and pays with one wave
 // of blocks sized by the list build's registers, which costs throughput once
 // the pair forces fill the GPU.  Measured, us per step, kernel by kernel ->
-// k_run: 250 beads 28 -> 16, 4,096 24 -> 16, 20,011 34 -> 26; 100,003 48 -> 46;
-// 1,048,576 241 -> 331.
+// k_run: 250 beads 28 -> 13, 4,096 24 -> 14, 20,011 34 -> 25, 100,003 47 -> 46,
+// a 200,000-bead melt 140 -> 154, 1,048,576 beads 238 -> 331.
 bool Engine::use_whole_steps() const {
-  constexpr uint32_t kWholeStepSlots = 65536;
+  constexpr uint32_t kWholeStepSlots = 131072;
   return use_graphs_ && v_.n_slots <= kWholeStepSlots && !(layout_fixed_ && v_.list_by_q != 0);
+}
+
+// Before lists are built: a context that nobody gave a layout or a schedule
+// takes the slot layout, whose global gathers mostly hit L1 and beat the staged
+// one on every size (1,048,576 beads: 0.174 against 0.233 ms a force
+// evaluation), and, when small, whole steps (true: nothing is left to tune).
+bool Engine::adopt_layout() {
+  if (tuning_fixed_ || tuned_) return whole_steps_;
+  if (v_.list_by_q != 0 && !layout_fixed_) {
+    v_.list_by_q = 0;
+    launch_.v = v_;
+    if (initialized_) relayout_list();
+  }
+  if (!use_whole_steps()) return false;
+  clear_graphs();
+  whole_steps_ = true;
+  launch_.lj_tpa = 4;
+  launch_.lj_unroll = 4;
+  launch_.lj_no_l1 = 1;
+  launch_.fuse_post = 1;
+  tuned_ = true;
+  return true;
 }
 
 // Times the force stage of a step (pair forces, bonded terms, second
@@ -151,24 +173,7 @@ bool Engine::use_whole_steps() const {
 void Engine::autotune() {
   TraceRange trace("beads.autotune");
   if (!initialized_) eval();
-  // The staged layout is kept only where it was asked for: the slot layout's
-  // global gathers mostly hit L1 and beat it on every size (1,048,576 beads:
-  // 0.174 against 0.233 ms a force evaluation).
-  if (v_.list_by_q != 0 && !layout_fixed_) {
-    v_.list_by_q = 0;
-    launch_.v = v_;
-    relayout_list();
-  }
-  if (use_whole_steps()) {
-    clear_graphs();
-    whole_steps_ = true;
-    launch_.lj_tpa = 4;
-    launch_.lj_unroll = 4;
-    launch_.lj_no_l1 = 1;
-    launch_.fuse_post = 1;
-    tuned_ = true;
-    return;
-  }
+  if (adopt_layout()) return;
   constexpr int kWarm = 1, kReps = 4;
   const bool log = [] {
     const char* e = std::getenv("BEADS_TUNE_LOG");
@@ -785,7 +790,6 @@ void Engine::d2h(void* dst, const void* src, size_t bytes, const char* what) {
 }
 
 void Engine::check_status() {
-  sync();
   d2h(h_state_, v_.rs, rep_.size() * sizeof(ReplicaState), "status download");
   for (uint32_t r = 0; r < rep_.size(); ++r) {
     const unsigned s = h_state_[r].status;
@@ -816,12 +820,25 @@ void Engine::check_status() {
   }
 }
 
+// Queues the download of the observables (into pinned memory): whoever waits
+// for the stream next has them.
+void Engine::queue_observables() {
+  cuda_check(cudaMemcpyAsync(h_obs_, v_.obs, rep_.size() * sizeof(ReplicaObs),
+                             cudaMemcpyDeviceToHost, stream_), "observables download");
+  obs_downloaded_ = true;
+}
+
 void Engine::eval() {
   TraceRange trace("beads.eval");
-  launch_apply_lambda(launch_);
-  launch_rebuild(launch_, true);
-  launch_forces(launch_, true, false);
-  launch_post(launch_, false, true);
+  if (adopt_layout()) {
+    launch_eval(launch_, run_);
+  } else {
+    flush_lambda();
+    launch_rebuild(launch_, true);
+    launch_forces(launch_, true, false);
+    launch_post(launch_, false, true);
+  }
+  queue_observables();
   check_status();
   initialized_ = true;
 }
@@ -973,6 +990,7 @@ bool Engine::run(uint64_t steps, uint64_t obs_every, const std::function<bool()>
   TraceRange trace("beads.run");
   if (!initialized_) eval();
   if (!tuned_ && !tuning_fixed_ && steps > 0) autotune();
+  if (steps > 0) obs_downloaded_ = false;
   const uint32_t n = n_replicas();
   bool last_obs = false;
   uint64_t remaining = steps;
@@ -1014,6 +1032,7 @@ bool Engine::run(uint64_t steps, uint64_t obs_every, const std::function<bool()>
                                  sizeof(ReplicaState), sizeof(unsigned), n,
                                  cudaMemcpyDeviceToHost, stream_),
                "status copy");
+    if (obs && remaining == chunk) queue_observables();
     cuda_check(cudaEventRecord(chunk_event_[k % kStatusRing], stream_), "event record");
     step_ += chunk;
     remaining -= chunk;
@@ -1036,7 +1055,14 @@ bool Engine::run(uint64_t steps, uint64_t obs_every, const std::function<bool()>
       }
     }
   }
-  check_status();
+  // Status bits stay set, so the last chunk's words hold every step's; one
+  // wait covers them and the observables queued before its event.
+  if (chunks == 0) {
+    check_status();
+  } else {
+    cuda_check(cudaEventSynchronize(chunk_event_[(chunks - 1) % kStatusRing]), "status wait");
+    if (chunk_failed(chunks - 1)) check_status();
+  }
   return last_obs;
 }
 
@@ -1075,7 +1101,9 @@ void Engine::minimize(uint32_t iterations, float dmax, float fref) {
   step_ = 0;
 }
 
-void Engine::flush_lambda() { launch_apply_lambda(launch_); }
+void Engine::flush_lambda() {
+  if (launch_.need_kinetic) launch_apply_lambda(launch_);  // else no scale is ever pending
+}
 
 double Engine::profile(int stage, uint32_t reps) {
   if (!initialized_) eval();
@@ -1164,8 +1192,7 @@ void Engine::list_stats(uint64_t* total, uint32_t* max_count) {
 }
 
 void Engine::observables(std::vector<beads_observables>& out) {
-  sync();
-  d2h(h_obs_, v_.obs, rep_.size() * sizeof(ReplicaObs), "observables download");
+  if (!obs_downloaded_) d2h(h_obs_, v_.obs, rep_.size() * sizeof(ReplicaObs), "observables download");
   convert_observables(h_obs_, out);
 }
 

@@ -87,6 +87,7 @@ class Engine {
   void minimize(uint32_t iterations, float dmax, float fref);
 
   void observables(std::vector<beads_observables>& out);
+  void queue_observables();
   void convert_observables(const ReplicaObs* raw, std::vector<beads_observables>& out) const;
   void state(uint32_t r, float* pos, float* vel, float* force, int32_t* img,
              uint32_t* tag_slot_order = nullptr, int32_t* type_slot = nullptr);
@@ -138,6 +139,7 @@ class Engine {
   // Whether steps run in one persistent kernel (run_kernel.cu) when the
   // schedule is not fixed by hand.
   bool use_whole_steps() const;
+  bool adopt_layout();
 
   // ---- adjoint (reverse-mode gradients of a trajectory; adjoint.cu) ----
   // Replaces the LJ eps/sigma tables of one replica (full n_types^2 tables).
@@ -228,6 +230,7 @@ class Engine {
   std::map<std::pair<uint32_t, bool>, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs_;
   std::map<uint32_t, std::pair<cudaGraph_t, cudaGraphExec_t>> replay_graphs_;
   ReplicaObs* h_obs_ = nullptr;        // pinned
+  bool obs_downloaded_ = false;        // h_obs_ holds (or will, after a wait) DeviceView::obs
   ReplicaState* h_state_ = nullptr;    // pinned
   // Status words of the last kStatusRing chunks (pinned, [kStatusRing][n_replicas]).
   // The run loop checks a chunk's words once the two chunks after it are

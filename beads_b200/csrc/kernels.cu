@@ -62,17 +62,7 @@ __global__ void k_decide(DeviceView v, cudaGraphConditionalHandle cond, int use_
 __global__ void k_force_rebuild_flags(DeviceView v, int count_build) {
   const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= v.n_replicas) return;
-  ReplicaState* st = &v.rs[r];
-  const ReplicaParams& p = v.rp[r];
-  st->need_rebuild = 1u;
-  if (count_build) {
-    st->builds += 1ull;
-    st->reorder_now =
-        (p.sort_every > 0u && (st->builds % p.sort_every) == 0ull) ? 1u : 0u;
-  } else {
-    st->reorder_now = 0u;
-  }
-  st->checks_since_build = 0u;
+  force_rebuild(v.rp[r], &v.rs[r], count_build != 0);
 }
 
 // rebuild 2: exclusive scan of the cell counts (the cell starts), in three

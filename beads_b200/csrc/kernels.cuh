@@ -9,7 +9,8 @@ namespace bb {
 // drift, wrap, displacement check, rebuild decision) -> rebuild chain (each
 // kernel returns at once for replicas that do not rebuild) -> pair forces ->
 // bonded forces -> post (half-kick, kinetic energy, observables, next lambda).
-enum PreMode : int { kPreVerlet = 0, kPreDescent = 1 };
+// kPreEval (run_kernel.cu only): no move, every list built, forces and totals.
+enum PreMode : int { kPreVerlet = 0, kPreDescent = 1, kPreEval = 2 };
 
 struct StepLaunch {
   DeviceView v;
@@ -98,6 +99,9 @@ constexpr int kRunBlocksPerSm = 7;  // resident blocks: the list build's registe
 void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables,
                 const RunRecord& rec = RunRecord{});
 void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps);
+// The evaluation of the current state: pending Berendsen scales applied, every
+// list built, forces, energies, virial and kinetic energy.
+void launch_eval(const StepLaunch& l, const RunView& rv);
 uint32_t run_scan_chunks(uint32_t total_cells);
 
 }  // namespace bb

@@ -249,8 +249,12 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
   for (uint32_t r = (gridDim.x - 1u - blockIdx.x) * kBlock + threadIdx.x; r < v.n_replicas;
        r += gridDim.x * kBlock) {
     ReplicaState* st = &v.rs[r];
-    if (kPre == kPreVerlet) count_checks(v.rp[r], st, since, step);
-    decide_replica<kPre>(v.rp[r], st, st->step + step + 1ull);
+    if (kPre == kPreEval) {
+      force_rebuild(v.rp[r], st, true);
+    } else {
+      if (kPre == kPreVerlet) count_checks(v.rp[r], st, since, step);
+      decide_replica<kPre>(v.rp[r], st, st->step + step + 1ull);
+    }
   }
   if (items == 0u) return grid_barrier(rv.ctl, &v.rs->status, target);  // launch-uniform
   if (!wide) {
@@ -349,12 +353,14 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
 }
 
 // kPre: velocity Verlet (drift, rebuild, forces and second half-kick per step)
-// or the capped descent (forces, move, rebuild per iteration).  kObs: energies
-// and virial of every step.
+// or the capped descent (forces, move, rebuild per iteration), or one
+// evaluation (rebuild, forces, totals).  kObs: energies and virial of every
+// step.
 template <int kPre, bool kObs, int kNt, bool kSmall>
 __global__ void __launch_bounds__(kBlock, kSmall ? kSmallBlocksPerSm : kRunBlocksPerSm)
 k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, float sd_fref) {
   constexpr bool kVerlet = kPre == kPreVerlet;
+  constexpr bool kEval = kPre == kPreEval;
   __shared__ RunShared sh;
   // The parameters and the LJ table of the replica at hand: after a barrier
   // they would come from L2 again.
@@ -363,7 +369,7 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
   __shared__ float lam_s;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t gthread = blockIdx.x * kBlock + threadIdx.x;
-  const bool kinetic = kVerlet && (kObs || rv.need_kinetic != 0);
+  const bool kinetic = kEval || (kVerlet && (kObs || rv.need_kinetic != 0));
   const bool bonded = v.has_bonded != 0;
   uint32_t target = 0, cur = 0xffffffffu;
   // Consecutive slot blocks and pair-force items per block: an item's
@@ -395,7 +401,7 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
   auto forces = [&](long long* ke, float4* vel) -> bool {
     for (uint32_t item = i0; item < i1; ++item) {
       enter(replica_of(item / kRunTpa));
-      lj_block<kObs, !kVerlet, kRunTpa, kSmall ? 8 : 4, true, kNt, true>(v, p, cur, item, table,
+      lj_block<kObs, kPre == kPreDescent, kRunTpa, kSmall ? 8 : 4, true, kNt, true>(v, p, cur, item, table,
                                                          kVerlet && !bonded, kinetic, ke, vel);
     }
     if (bonded) {
@@ -417,13 +423,14 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
          r += gridDim.x * kBuildWarps) {
       const double kin = kinetic ? bucket_kinetic(ke, r, lane) : 0.0;
       if (lane != 0u) continue;
-      const double l = kinetic ? berendsen_lambda(v.rp[r], kin) : 1.0;
+      const double l = kVerlet && kinetic ? berendsen_lambda(v.rp[r], kin) : 1.0;
       if (rec.lam) {
         rec.lam[(size_t)(rec.k0 + s + 1u) * v.n_replicas + r] = l;
         rec.kin[(size_t)(rec.k0 + s + 1u) * v.n_replicas + r] = kin;
       }
       if (kObs) {
-        const ReplicaObs o = take_observables(&v.rs[r], v.rs[r].step + s + 1ull, kin, l);
+        const ReplicaObs o = take_observables(&v.rs[r], v.rs[r].step + (kEval ? 0u : s + 1u), kin,
+                                                l);
         if (rec.obs) rec.obs[(size_t)s * v.n_replicas + r] = o;
         if (s + 1u == n_steps) v.obs[r] = o;
       }
@@ -431,7 +438,29 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
   };
 
   uint32_t since = 0;  // steps whose checks are counted
-  for (uint32_t s = 0; s < n_steps; ++s) {
+  if (kEval) {
+    // Own velocities: the pending scale, and their kinetic energy.
+    for (uint32_t b = b0; b < b1; ++b) {
+      const uint32_t r = replica_of(b);
+      enter(r);
+      const uint32_t i = b * kBlock + threadIdx.x;
+      const bool real = (i - p.atom_begin) < p.n_atoms;
+      const float lam = (float)v.rs[r].lambda;
+      float4 u = real ? v.vel[i] : make_float4(0.f, 0.f, 0.f, 1.f);
+      if (real && lam != 1.0f) {
+        u.x = __fmul_rn(u.x, lam);
+        u.y = __fmul_rn(u.y, lam);
+        u.z = __fmul_rn(u.z, lam);
+        v.vel[i] = u;
+      }
+      post_partial(v.ke_part, &v.rs[r], r, real,
+                   post_slot_vm(v, p, &v.rs[r], i, real, false, true, u, 0.f, 0.f, 0.f));
+    }
+    if (!run_rebuild<kPre>(v, rv, rec, sh, b0, b1, 0u, 0u, target)) return;
+    if (!forces(nullptr, nullptr)) return;
+    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+  }
+  for (uint32_t s = 0; !kEval && s < n_steps; ++s) {
     long long* ke = (s & 1u) ? rv.ke_odd : v.ke_part;
     long long* ke_other = (s & 1u) ? v.ke_part : rv.ke_odd;
     if (!kVerlet) {
@@ -488,7 +517,7 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
       if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
     }
   }
-  if (kVerlet) {
+  if (kVerlet || kEval) {
     long long* ke = (n_steps & 1u) ? v.ke_part : rv.ke_odd;  // of the last step
     if (kObs || rec.lam) epilogue(n_steps - 1u, ke);
     for (uint32_t r = blockIdx.x * kBuildWarps + warp; r < v.n_replicas;
@@ -502,13 +531,13 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
       }
       if (lane == 0u) {
         ReplicaState* st = &v.rs[r];
-        if (since < n_steps) {
+        if (kVerlet && since < n_steps) {
           count_checks(v.rp[r], st, since, n_steps);
           st->need_rebuild = 0u;
           st->reorder_now = 0u;
         }
-        st->lambda = kinetic ? berendsen_lambda(v.rp[r], kin) : 1.0;
-        st->step += n_steps;
+        st->lambda = kVerlet && kinetic ? berendsen_lambda(v.rp[r], kin) : 1.0;
+        if (kVerlet) st->step += n_steps;
         if (kinetic) st->last_kinetic = kin;
       }
     }
@@ -584,6 +613,10 @@ void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool o
 
 void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
   launch_one<kPreDescent, false, 0>(l, rv, RunRecord{}, n_steps);
+}
+
+void launch_eval(const StepLaunch& l, const RunView& rv) {
+  launch_one<kPreEval, true, 0>(l, rv, RunRecord{}, 1);
 }
 
 uint32_t run_scan_chunks(uint32_t total_cells) {

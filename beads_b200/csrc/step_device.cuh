@@ -101,9 +101,22 @@ __device__ __forceinline__ void pre_block(const DeviceView& v, const ReplicaPara
 template <int kMode>
 __device__ __forceinline__ bool needs_rebuild(const ReplicaParams& p, const ReplicaState* st,
                                               unsigned long long phys) {
+  if (kMode == kPreEval) return true;
   if (st->status & (kStatusNonFinite | kStatusFixedOverflow)) return false;
   if (kMode == kPreVerlet && p.skin == 0.0f) return true;
   return st->exceeded != 0u && is_check_step<kMode>(p, phys);
+}
+
+// Marks one replica for a rebuild (initial build / explicit eval).
+__device__ __forceinline__ void force_rebuild(const ReplicaParams& p, ReplicaState* st,
+                                              bool count_build) {
+  st->need_rebuild = 1u;
+  st->reorder_now = 0u;
+  if (count_build) {
+    st->builds += 1ull;
+    st->reorder_now = (p.sort_every > 0u && (st->builds % p.sort_every) == 0ull) ? 1u : 0u;
+  }
+  st->checks_since_build = 0u;
 }
 
 // The rebuild decision of one replica for step `phys` (neighbor_system.cpp:79-105).
