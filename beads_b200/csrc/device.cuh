@@ -184,6 +184,7 @@ struct DeviceView {
   uint32_t* cell_of_slot;
   uint32_t* cell_count;
   uint32_t* cell_cursor;
+  uint32_t* big_cells;       // cells of sparse replicas too big for a thread's sort (count)
   uint32_t* cell_start;
   uint32_t* cell_atoms;
   // neighbour list

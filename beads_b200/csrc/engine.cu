@@ -646,6 +646,7 @@ void Engine::upload_static(uint32_t n, const beads_system_desc* systems,
   v.cell_of_slot = dalloc<uint32_t>(S);
   v.cell_count = dalloc<uint32_t>(C);
   v.cell_cursor = dalloc<uint32_t>(C);
+  v.big_cells = dalloc<uint32_t>(1);
   v.cell_start = dalloc<uint32_t>(static_cast<size_t>(C) + n);
   v.cell_atoms = dalloc<uint32_t>(S);
   v.nbr_count = dalloc<uint32_t>(S);

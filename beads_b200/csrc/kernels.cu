@@ -24,6 +24,7 @@
 #include "device_util.cuh"
 #include "step_device.cuh"
 
+#include <algorithm>
 #include <cstdio>
 #include <stdexcept>
 #include <string>
@@ -122,7 +123,10 @@ __device__ __forceinline__ void for_chain_blocks(const DeviceView& v) {
 }
 
 __global__ void __launch_bounds__(kBlock) k_bin(DeviceView v) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) *v.chain_launches += 1ull;  // launches of the chain
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *v.chain_launches += 1ull;  // launches of the chain
+    *v.big_cells = 0u;
+  }
   for_chain_blocks<bin_block>(v);
 }
 
@@ -257,18 +261,29 @@ __global__ void __launch_bounds__(kBlock) k_scatter(DeviceView v) {
 
 __global__ void __launch_bounds__(kBlock) k_cellsort_sparse(DeviceView v) {
   const uint32_t w = blockIdx.x * kBlock + threadIdx.x;
-  if (w < v.work_start[v.n_replicas]) sort_cell_sparse(v, w);
+  // The cells left over are listed for k_cellsort (the cursors are free once
+  // the slots are scattered).
+  if (w < v.work_start[v.n_replicas] && !sort_cell_sparse(v, w)) {
+    v.cell_cursor[atomicAdd(v.big_cells, 1u)] = w;
+  }
 }
 
 // Warp w sorts work item w (k_scan): the warps past the cells of the
-// rebuilding replicas return after one load.
-__global__ void __launch_bounds__(kBlock) k_cellsort(DeviceView v) {
+// rebuilding replicas return after one load.  listed: every replica is sparse,
+// and a few blocks walk the cells k_cellsort_sparse listed instead (a warp per
+// cell that finds nothing to do took ~12 us of a 200,000-bead melt's rebuild).
+__global__ void __launch_bounds__(kBlock) k_cellsort(DeviceView v, int listed) {
   __shared__ uint32_t sort_keys[kBlock / 32][kSortRankMax];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t w = blockIdx.x * (kBlock / 32) + warp;
-  if (w >= v.work_start[v.n_replicas]) return;  // warp-uniform
-  const uint32_t r = work_replica(v, w);
-  sort_cell(v, v.rp[r], w - v.work_start[r], lane, sort_keys[warp]);
+  const uint32_t first = blockIdx.x * (kBlock / 32) + warp;
+  const uint32_t n = listed ? *v.big_cells : v.work_start[v.n_replicas];
+  const uint32_t step = listed ? gridDim.x * (kBlock / 32) : n;
+  for (uint32_t k = first; k < n; k += step) {  // warp-uniform
+    const uint32_t w = listed ? v.cell_cursor[k] : k;
+    const uint32_t r = work_replica(v, w);
+    sort_cell(v, v.rp[r], w - v.work_start[r], lane, sort_keys[warp]);
+    __syncwarp();
+  }
 }
 
 __global__ void __launch_bounds__(kBlock) k_reorder_gather(DeviceView v) {
@@ -302,7 +317,7 @@ __global__ void __launch_bounds__(kBlock, 7) k_build(DeviceView v, uint32_t part
 }
 
 template <bool kExcl, bool kByQ>
-__global__ void __launch_bounds__(kBlock) k_build_sparse(DeviceView v) {
+__global__ void __launch_bounds__(kBlock, kByQ ? 1 : 12) k_build_sparse(DeviceView v) {
   __shared__ StageLayout lay;
   build_sparse_block<kExcl, kByQ>(v, blockIdx.x, lay);
 }
@@ -713,7 +728,12 @@ void launch_rebuild(const StepLaunch& l, bool force_all, bool count_build) {
     k_cellsort_sparse<<<(l.v.total_cells + kBlock - 1) / kBlock, kBlock, 0, l.stream>>>(l.v);
     check_launch("cellsort sparse");
   }
-  k_cellsort<<<(l.v.total_cells + kBlock / 32 - 1) / (kBlock / 32), kBlock, 0, l.stream>>>(l.v);
+  const uint32_t sort_blocks = (l.v.total_cells + kBlock / 32 - 1) / (kBlock / 32);
+  if (l.any_dense) {
+    k_cellsort<<<sort_blocks, kBlock, 0, l.stream>>>(l.v, 0);
+  } else {
+    k_cellsort<<<std::min(sort_blocks, 148u), kBlock, 0, l.stream>>>(l.v, 1);
+  }
   check_launch("cellsort");
   k_reorder_gather<<<sg, kBlock, 0, l.stream>>>(l.v);
   check_launch("reorder_gather");

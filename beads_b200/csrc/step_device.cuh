@@ -300,16 +300,17 @@ __device__ __forceinline__ void sort_cell(const DeviceView& v, const ReplicaPara
 
 // Cells of sparse replicas (k_build_sparse) with at most kSortThreadMax
 // members: one thread per work item sorts its cell's slots in registers
-// (insertion sort) and gathers their positions; k_cellsort sorts the rest.
-__device__ __forceinline__ void sort_cell_sparse(const DeviceView& v, uint32_t w) {
+// (insertion sort) and gathers their positions; false for the cells left to
+// k_cellsort.
+__device__ __forceinline__ bool sort_cell_sparse(const DeviceView& v, uint32_t w) {
   const uint32_t r = work_replica(v, w);
   const ReplicaParams& p = v.rp[r];
-  if (!p.sparse) return;
+  if (!p.sparse) return false;
   const uint32_t c = w - v.work_start[r];
   const uint32_t s0 = v.cell_start[p.start_base + c];
   const uint32_t s1 = v.cell_start[p.start_base + c + 1];
   const uint32_t n = s1 - s0;
-  if (n > kSortThreadMax) return;
+  if (n > kSortThreadMax) return false;
   uint32_t key[kSortThreadMax];
 #pragma unroll
   for (uint32_t k = 0; k < kSortThreadMax; ++k) key[k] = k < n ? v.cell_atoms[s0 + k] : 0xffffffffu;
@@ -330,6 +331,7 @@ __device__ __forceinline__ void sort_cell_sparse(const DeviceView& v, uint32_t w
       v.pos2[s0 + k] = v.pos[key[k]];
     }
   }
+  return true;
 }
 
 // rebuild 5/6: physical reorder into cell order (every sort_every builds).
@@ -806,6 +808,8 @@ __device__ __forceinline__ void build_cell(const DeviceView& v, const ReplicaPar
 // so the lists (order included) are the ones k_build writes.  A block is 128
 // consecutive cell-order rows: one stage group in a staged context.  kByQ
 // as for k_build.
+constexpr uint32_t kSparseBatch = 2;
+
 template <bool kExcl, bool kByQ>
 __device__ __forceinline__ void build_sparse_block(const DeviceView& v, uint32_t b,
                                                    StageLayout& lay) {
@@ -847,37 +851,44 @@ __device__ __forceinline__ void build_sparse_block(const DeviceView& v, uint32_t
   // One segment: cell-order run [q0, q1), periodic shift (sx, sy, sz) for the
   // shifted form, entry offset `delta` (stage index = q + delta) in a staged
   // group.
+  // Two candidates' positions are loaded before any is tested (a thread's
+  // walk waits on its loads); slots only of the candidates in range.
   auto walk = [&](uint32_t q0, uint32_t q1, float sx, float sy, float sz, uint32_t delta) {
-    for (uint32_t qc = q0; qc < q1; ++qc) {
-      const uint32_t j = v.cell_atoms[qc];
-      const float4 x = v.pos2[qc];
-      float dx, dy, dz;
-      if (form == kBuildMinImage) {
-        dx = ref_delta(xi.x, x.x, p.len[0], p.half[0]);
-        dy = ref_delta(xi.y, x.y, p.len[1], p.half[1]);
-        dz = ref_delta(xi.z, x.z, p.len[2], p.half[2]);
-      } else {
-        dx = __fsub_rn(xi.x, x.x);
-        dy = __fsub_rn(xi.y, x.y);
-        dz = __fsub_rn(xi.z, x.z);
-        if (form == kBuildShifted) {
-          dx = __fadd_rn(dx, sx);
-          dy = __fadd_rn(dy, sy);
-          dz = __fadd_rn(dz, sz);
-        }
-      }
-      bool ok = !(norm2(dx, dy, dz) > cut) && j != i;
-      if (kExcl) {
-        ok = ok && j != ex0.x && j != ex0.y && j != ex0.z && j != ex0.w;
-        if (ok && ex0.w != 0xffffffffu) {
-#pragma unroll 1
-          for (uint32_t e = 1; e < v.excl_cap / 4u; ++e) {
-            const uint4 x = ex[e];
-            ok = ok && j != x.x && j != x.y && j != x.z && j != x.w;
+    for (uint32_t qb = q0; qb < q1; qb += kSparseBatch) {
+      float4 x[kSparseBatch];
+#pragma unroll
+      for (uint32_t u = 0; u < kSparseBatch; ++u) x[u] = v.pos2[min(qb + u, q1 - 1u)];
+#pragma unroll
+      for (uint32_t u = 0; u < kSparseBatch; ++u) {
+        const uint32_t qc = qb + u;
+        float dx, dy, dz;
+        if (form == kBuildMinImage) {
+          dx = ref_delta(xi.x, x[u].x, p.len[0], p.half[0]);
+          dy = ref_delta(xi.y, x[u].y, p.len[1], p.half[1]);
+          dz = ref_delta(xi.z, x[u].z, p.len[2], p.half[2]);
+        } else {
+          dx = __fsub_rn(xi.x, x[u].x);
+          dy = __fsub_rn(xi.y, x[u].y);
+          dz = __fsub_rn(xi.z, x[u].z);
+          if (form == kBuildShifted) {
+            dx = __fadd_rn(dx, sx);
+            dy = __fadd_rn(dy, sy);
+            dz = __fadd_rn(dz, sz);
           }
         }
-      }
-      if (ok) {
+        if (qc >= q1 || qc == q || norm2(dx, dy, dz) > cut) continue;
+        const uint32_t j = v.cell_atoms[qc];
+        if (kExcl) {
+          bool ok = j != ex0.x && j != ex0.y && j != ex0.z && j != ex0.w;
+          if (ok && ex0.w != 0xffffffffu) {
+#pragma unroll 1
+            for (uint32_t e = 1; e < v.excl_cap / 4u; ++e) {
+              const uint4 y = ex[e];
+              ok = ok && j != y.x && j != y.y && j != y.z && j != y.w;
+            }
+          }
+          if (!ok) continue;
+        }
         if (cnt < cap) row[(size_t)cnt * kGroup] = staged_group ? qc + delta : j;
         ++cnt;
       }
