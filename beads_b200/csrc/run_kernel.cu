@@ -596,23 +596,30 @@ void launch_one(const StepLaunch& l, const RunView& rv, const RunRecord& rec, ui
   }
 }
 
+// The LJ table specialisation of the batch: its coefficients in registers for
+// one or two types.
+template <int kPre, bool kObs>
+void launch_types(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uint32_t n_steps) {
+  switch (l.lj_types) {
+    case 1: launch_one<kPre, kObs, 1>(l, rv, rec, n_steps); break;
+    case 2: launch_one<kPre, kObs, 2>(l, rv, rec, n_steps); break;
+    default: launch_one<kPre, kObs, 0>(l, rv, rec, n_steps); break;
+  }
+}
+
 }  // namespace
 
 void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables,
                 const RunRecord& rec) {
   if (observables) {
-    launch_one<kPreVerlet, true, 0>(l, rv, rec, n_steps);
-  } else if (l.lj_types == 1) {
-    launch_one<kPreVerlet, false, 1>(l, rv, rec, n_steps);
-  } else if (l.lj_types == 2) {
-    launch_one<kPreVerlet, false, 2>(l, rv, rec, n_steps);
+    launch_types<kPreVerlet, true>(l, rv, rec, n_steps);
   } else {
-    launch_one<kPreVerlet, false, 0>(l, rv, rec, n_steps);
+    launch_types<kPreVerlet, false>(l, rv, rec, n_steps);
   }
 }
 
 void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
-  launch_one<kPreDescent, false, 0>(l, rv, RunRecord{}, n_steps);
+  launch_types<kPreDescent, false>(l, rv, RunRecord{}, n_steps);
 }
 
 void launch_eval(const StepLaunch& l, const RunView& rv) {
