@@ -139,8 +139,9 @@ void Engine::tuning(int* tpa, int* fuse_post, int* unroll, int* no_l1, int* auto
 // the pair forces fill the GPU.  Measured, us per step, kernel by kernel ->
 // k_run: 250 beads 28 -> 13, 4,096 24 -> 14, 20,011 34 -> 25, 100,003 47 -> 46,
 // a 200,000-bead melt 140 -> 154, 1,048,576 beads 238 -> 331.
+constexpr uint32_t kWholeStepSlots = 131072;
+
 bool Engine::use_whole_steps() const {
-  constexpr uint32_t kWholeStepSlots = 131072;
   return use_graphs_ && v_.n_slots <= kWholeStepSlots && !(layout_fixed_ && v_.list_by_q != 0);
 }
 
@@ -1069,22 +1070,31 @@ bool Engine::run(uint64_t steps, uint64_t obs_every, const std::function<bool()>
 
 void Engine::minimize(uint32_t iterations, float dmax, float fref) {
   TraceRange trace("beads.minimize");
-  // The descent steps in k_run, on slot rows; a staged context goes back to
-  // its layout afterwards (its next evaluation builds the list again).
-  const int by_q = v_.list_by_q;
-  v_.list_by_q = 0;
-  launch_.v = v_;
   StepLaunch l = launch_;
   l.sd_dmax = dmax;
   l.sd_fref = fref;
-  constexpr uint32_t kDescentChunk = 64;
-  launch_rebuild(l, true);
-  for (uint32_t it = 0; it < iterations; it += kDescentChunk) {
-    launch_descent(l, run_, std::min(kDescentChunk, iterations - it));
+  if (use_graphs_ && v_.n_slots <= kWholeStepSlots) {
+    // In k_run, on slot rows; a staged context goes back to its layout
+    // afterwards (its next evaluation builds the list again).
+    const int by_q = v_.list_by_q;
+    v_.list_by_q = 0;
+    launch_.v = l.v = v_;
+    constexpr uint32_t kDescentChunk = 64;
+    launch_rebuild(l, true);
+    for (uint32_t it = 0; it < iterations; it += kDescentChunk) {
+      launch_descent(l, run_, std::min(kDescentChunk, iterations - it));
+    }
+    sync();
+    v_.list_by_q = by_q;
+    launch_.v = v_;
+  } else {
+    launch_rebuild(l, true);
+    for (uint32_t it = 0; it < iterations; ++it) {
+      launch_forces(l, false, true);
+      launch_pre(l, kPreDescent);
+      launch_rebuild(l, false);
+    }
   }
-  sync();
-  v_.list_by_q = by_q;
-  launch_.v = v_;
   // The descent is set-up work: reset counters so a following run starts
   // like a fresh one.
   check_status();

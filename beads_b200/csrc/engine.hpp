@@ -73,12 +73,14 @@ class Engine {
   // Advance `steps`; observables on multiples of obs_every (0 = never).
   // Returns true if the last step was an observable step.
   //
-  // The steps run as captured chunks of at most 16.  After launching chunk
-  // k the host reads the status words that chunk k - 1 left (a pinned copy
-  // queued behind it, so the device keeps chunk k to work on) and raises the
-  // error of a replica whose list overflowed, whose energy left the
-  // fixed-point range or whose velocities became non-finite: at most one
-  // chunk after the step that failed.  `poll`, when given, is called at the
+  // The steps run as chunks of at most 16, one launch of k_run or one captured
+  // graph each.  After launching chunk k the host reads the status words that
+  // chunk k - 2 left (a pinned copy queued behind it, so the device keeps two
+  // chunks to work on) and raises the error of a replica whose list overflowed,
+  // whose energy left the fixed-point range or whose velocities became
+  // non-finite: at most two chunks after the step that failed.  The end of a
+  // run waits once, for the last chunk's words and the observables queued
+  // before them.  `poll`, when given, is called at the
   // first chunk boundary at or after every `poll_every` steps; a true return
   // stops the run with std::runtime_error("interrupted") once the queued
   // chunks have drained.
@@ -105,8 +107,10 @@ class Engine {
   void debug_neighbors(uint32_t r, uint32_t cap, uint32_t* counts, uint32_t* partners);
   // Pair forces from shared-memory cell tiles (list rows by cell order, stage
   // indices as entries) or from global gathers (rows by slot, slot entries).
-  // Contexts start staged when some replica qualifies; switching rebuilds the
-  // list before the next force evaluation.  Results are the same bits.
+  // Contexts start staged when some replica qualifies and leave that layout at
+  // their first evaluation unless it was asked for (adopt_layout); switching
+  // rebuilds the list before the next force evaluation.  Results are the same
+  // bits.
   void set_list_staged(bool staged);
   bool list_staged() const { return v_.list_by_q != 0; }
   void debug_neighbors_staged(uint32_t r, uint32_t cap, uint32_t* counts, uint32_t* partners);
@@ -123,16 +127,18 @@ class Engine {
   // Kernels one MD step launches under the current schedule, and the
   // kernels of one rebuild chain when that chain runs only on rebuild steps
   // (0 when every step launches it: no conditional graph node).  Counted
-  // as the kernel nodes of one captured step; nothing is executed.
+  // as the kernel nodes of one captured step, also where steps run in k_run;
+  // nothing is executed.
   void launch_counts(uint32_t& per_step, uint32_t& per_chain);
   void check_status();
   // Kernel schedule of the step: threads per particle of the pair-force
   // kernel (1, 2 or 4), its batch depth (4 or 8 list entries in flight per
   // thread), whether its list loads bypass L1, and whether the second
   // half-kick runs inside the last force kernel.  Every choice gives bit-identical results.  tpa = 0 hands
-  // the choice back to the autotuner, which times every candidate on this
-  // batch at the first run (velocities and step state restored) and keeps
-  // the fastest.
+  // the choice back to the engine: contexts of up to 131,072 slots then step
+  // in k_run, for larger ones the autotuner times the candidates on this batch
+  // at the first run (velocities and step state restored) and keeps the
+  // fastest.
   void set_tuning(int tpa, int fuse_post, int unroll, int no_l1);
   void tuning(int* tpa, int* fuse_post, int* unroll, int* no_l1, int* autotuned) const;
   void autotune();
@@ -218,7 +224,7 @@ class Engine {
   bool staged_ = false;                // some replica stages its pair forces
   uint32_t stage_cap_ = 0;             // stage entries per group (k_lj_staged)
   bool tuning_fixed_ = false;          // set_tuning() with an explicit choice
-  bool layout_fixed_ = false;          // set_list_staged() called: the autotuner keeps the layout
+  bool layout_fixed_ = false;          // set_list_staged() called: the layout stays
   bool any_sparse_ = false, any_dense_ = false;  // list build forms in use (k_build_sparse / k_build)
   float4* relayout_pos_ = nullptr;     // relayout_list save buffers (allocated at first use)
   int4* relayout_img_ = nullptr;

@@ -295,7 +295,8 @@ class Engine:
     def set_list_staged(self, staged: bool) -> None:
         """Pair forces from shared-memory cell tiles (True) or global gathers
         (False); the same bits either way (beads_set_list_layout).  Once set,
-        the autotuner keeps this layout instead of timing both."""
+        this layout is kept; a context without a call (and without a schedule
+        fixed by hand) takes the slot layout at its first evaluation."""
         _lib.check(self._lib.beads_set_list_layout(self._h, 1 if staged else 0))
 
     def list_staged(self) -> bool:

@@ -292,8 +292,9 @@ BEADS_API int beads_get_tuning(beads_ctx* ctx, int32_t* schedule);
  * pair-force kernel reads every neighbour position.  Slot layout (0): rows
  * and entries by slot, positions gathered from global memory.  The choice
  * never changes a result; switching rebuilds the list before the next force
- * evaluation.  Without a call the autotuner times both layouts at the first
- * run and keeps the faster; after a call it keeps the layout set here.
+ * evaluation.  A context without a call, and without a schedule fixed by hand,
+ * takes the slot layout at its first evaluation (the faster one at every size);
+ * after a call it keeps the layout set here.
  * beads_get_list_layout reports 0 when no replica can stage.
  * No reference counterpart (the reference keeps one slot-major list,
  * neighbor_list.cuh:12-71). */
@@ -353,8 +354,11 @@ BEADS_API int beads_counters(beads_ctx* ctx, uint32_t replica, uint64_t* counter
  * (counters[3] of beads_counters counts those runs).  *per_rebuild_chain is 0
  * when every step launches the chain itself (no conditional graph node, or
  * graphs switched off with BEADS_GRAPHS=0); *per_step then includes it.
- * Counted as the kernel nodes of one captured step; nothing runs.  No
- * counterpart in the reference (measurement). */
+ * Counted as the kernel nodes of one captured step; nothing runs.  A context of
+ * up to 131,072 particle slots whose schedule nobody fixed does not step that
+ * way: it takes up to 16 steps, rebuilds included, per launch of one kernel,
+ * and the counts are those of the steps it would capture.  No counterpart in
+ * the reference (measurement). */
 BEADS_API int beads_launch_counts(beads_ctx* ctx, uint32_t* per_step,
                                   uint32_t* per_rebuild_chain);
 
