@@ -394,22 +394,31 @@ def execute_simulation(spec: Mapping[str, Any]) -> None:
     rd.dynamics = ctypes.pointer(parsed.dd)
     rd.thermostat_name = parsed.thermostat_name.encode()
     rd.exclusion_policy = parsed.exclusion_policy.encode()
-    interrupted = []
+    raised: list[BaseException] = []
 
-    def poll(_user) -> int:
+    def polls():
         # The reference checks PyErr_CheckSignals between steps (module.cpp:29-34).
-        try:
-            if ctypes.pythonapi.PyErr_CheckSignals() != 0:
-                interrupted.append(True)
-                return 1
-        except KeyboardInterrupt:
-            interrupted.append(True)
-            return 1
-        return 0
+        # Each poll resumes this generator inside the try: Python runs a pending
+        # signal's handler as soon as a frame starts, which in a plain function
+        # is before its first statement, where ctypes would drop the exception.
+        answer = 0
+        while True:
+            try:
+                yield answer
+                answer = 1 if ctypes.pythonapi.PyErr_CheckSignals() != 0 else answer
+            except GeneratorExit:
+                raise
+            except BaseException as exc:
+                raised.append(exc)
+                answer = 1
 
-    callback = _lib.INTERRUPT_FN(poll)
+    poller = polls()
+    next(poller)
+    callback = _lib.INTERRUPT_FN(poller.send)
     rd.interrupt = callback
     status = L.beads_execute(ctypes.byref(rd))
-    if status == _lib.ERR_INTERRUPTED or interrupted:
+    if raised:
+        raise raised[0]
+    if status == _lib.ERR_INTERRUPTED:
         raise KeyboardInterrupt
     _lib.check(status)
