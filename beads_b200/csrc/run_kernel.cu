@@ -371,6 +371,9 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
   const uint32_t gthread = blockIdx.x * kBlock + threadIdx.x;
   const bool kinetic = kEval || (kVerlet && (kObs || rv.need_kinetic != 0));
   const bool bonded = v.has_bonded != 0;
+  // A launch queued behind one whose barrier ran out finds the counts in
+  // disorder (the host rearms them when it reports the error).
+  if (__ldcg(&v.rs->status) & kStatusStalled) return;
   uint32_t target = 0, cur = 0xffffffffu;
   // Consecutive slot blocks and pair-force items per block: an item's
   // neighbours are mostly those of the item before it.

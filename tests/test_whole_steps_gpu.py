@@ -51,6 +51,13 @@ CASES = {
                                        thermostat=(1.2, 1.0))],
     "no_skin": lambda: [_fluid(300, (7.0, 7.0, 7.0), cutoff_buffer=0.0)],
     "sparse_gas": lambda: [_fluid(500, (40.0, 41.0, 39.0), seed=4)],
+    # more cells than 24 per warp of the launch: lists a thread per particle
+    "dilute_gas": lambda: [_fluid(700, (95.0, 95.0, 95.0), seed=7, thermostat=(1.0, 1.0))],
+    # more replicas than a block has threads, one of them of more cells than a
+    # block scans
+    "many_replicas": lambda: [_fluid(40 + k, (6.5, 6.5, 6.5), seed=k,
+                                     thermostat=(1.0, 1.0) if k % 3 else None)
+                              for k in range(140)] + [_fluid(500, (40.0, 41.0, 39.0), seed=4)],
     "melt": lambda: [workloads.polymer_melt(n_chains=20, beads=50, seed=4, max_neighbors=96)],
     "batch": lambda: [_fluid(1, (6.0, 6.0, 6.0)), _fluid(700, (9.0, 9.0, 9.0), seed=2),
                       workloads.polymer_melt(n_chains=10, beads=30, seed=5, max_neighbors=96)]
