@@ -748,8 +748,10 @@ void launch_rebuild(const StepLaunch& l, bool force_all, bool count_build) {
   // the last wave nearly empty: in a batch only the rebuilding replicas' cells
   // count, a fraction of the grid.  Measured with 1 / 2 / 3 / 4 shares: 128
   // replicas (832,000 beads) 491 / 412 / 400 / 402 us a step, 100,003 beads
-  // 46.9 / 46.6 / 47.1 / 47.2, 1,048,576 beads 238 / 240 / 245 / 250.
-  const uint32_t parts = l.v.n_replicas > 1u ? 3u : l.v.total_cells < 16384u ? 2u : 1u;
+  // 46.9 / 46.6 / 47.1 / 47.2, 1,048,576 beads 238 / 240 / 245 / 250; 512
+  // replicas (3.3 M beads, some waves of rebuilding cells) 1242 / - / 1257.
+  const uint32_t parts = l.v.n_replicas > 1u ? (l.v.total_cells < 65536u ? 3u : 1u)
+                         : l.v.total_cells < 16384u ? 2u : 1u;
   const uint32_t bg = (l.v.total_cells * parts + kBuildWarps - 1) / kBuildWarps;
 #define BB_BUILD(excl, q)                                                                  \
   do {                                                                                     \
