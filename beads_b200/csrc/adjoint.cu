@@ -198,11 +198,12 @@ struct AdjCoeff {
   float pad;
 };
 
-// Warp total of fixed-point contributions (frac words in [0, 2^32)): 16-bit
-// pieces through the 32-bit integer reduction, exact modulo 2^64.
+// Warp total of fixed-point contributions (frac words in [0, 2^32], see
+// to_fixed): pieces of 16 bits, and the 17 bits above a fraction's lower half,
+// through the 32-bit integer reduction, exact modulo 2^64.
 __device__ __forceinline__ Fixed warp_sum(Fixed f) {
   const unsigned long long w = (unsigned long long)f.whole;
-  const uint32_t lo = (uint32_t)f.frac;
+  const unsigned long long q = (unsigned long long)f.frac;
   unsigned long long whole = 0ull;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -210,8 +211,8 @@ __device__ __forceinline__ Fixed warp_sum(Fixed f) {
              << (16 * k);
   }
   const unsigned long long frac =
-      (unsigned long long)__reduce_add_sync(kFull, lo & 0xffffu) +
-      ((unsigned long long)__reduce_add_sync(kFull, lo >> 16) << 16);
+      (unsigned long long)__reduce_add_sync(kFull, (uint32_t)q & 0xffffu) +
+      ((unsigned long long)__reduce_add_sync(kFull, (uint32_t)(q >> 16)) << 16);
   return Fixed{(long long)whole, (long long)frac};
 }
 

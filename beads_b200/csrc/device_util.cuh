@@ -13,7 +13,9 @@ namespace bb {
 constexpr unsigned kFull = 0xffffffffu;
 
 // One slot's contribution to a fixed-point total: floor(v) and the fraction
-// v - floor(v) (exact in double) truncated to units of 2^-32.
+// v - floor(v) truncated to units of 2^-32.  The difference is rounded to
+// double, so for a negative v of at most 2^-54 in size it is 1 and frac is
+// 2^32: sums of frac words have to keep that carry.
 struct Fixed {
   long long whole;
   long long frac;
