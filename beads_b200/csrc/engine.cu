@@ -1074,19 +1074,31 @@ void Engine::minimize(uint32_t iterations, float dmax, float fref) {
   l.sd_dmax = dmax;
   l.sd_fref = fref;
   if (use_graphs_ && v_.n_slots <= kWholeStepSlots) {
-    // In k_run, on slot rows; a staged context goes back to its layout
-    // afterwards (its next evaluation builds the list again).
+    // In k_run, on slot rows.  A context with a staged layout asked for by hand
+    // leaves it for the descent; the list that is left is then laid out again,
+    // so that list and layout agree between calls.
+    adopt_layout();
     const int by_q = v_.list_by_q;
     v_.list_by_q = 0;
     launch_.v = l.v = v_;
-    constexpr uint32_t kDescentChunk = 64;
-    launch_rebuild(l, true);
-    for (uint32_t it = 0; it < iterations; it += kDescentChunk) {
-      launch_descent(l, run_, std::min(kDescentChunk, iterations - it));
+    try {
+      constexpr uint32_t kDescentChunk = 64;
+      launch_rebuild(l, true);
+      for (uint32_t it = 0; it < iterations; it += kDescentChunk) {
+        launch_descent(l, run_, std::min(kDescentChunk, iterations - it));
+      }
+      sync();
+    } catch (...) {
+      v_.list_by_q = by_q;
+      launch_.v = v_;
+      initialized_ = false;
+      throw;
     }
-    sync();
-    v_.list_by_q = by_q;
-    launch_.v = v_;
+    if (by_q != 0) {
+      v_.list_by_q = by_q;
+      launch_.v = v_;
+      relayout_list();
+    }
   } else {
     launch_rebuild(l, true);
     for (uint32_t it = 0; it < iterations; ++it) {

@@ -1,0 +1,46 @@
+"""The neighbour list and the layout a context says it has agree between calls."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from beads_b200 import workloads
+from beads_b200.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _lists(eng):
+    counts, partners = eng.debug_neighbors()
+    return counts, [np.sort(row[:c]) for row, c in zip(partners, counts)]
+
+
+@pytest.mark.parametrize("hand", ["", "schedule", "staged"])
+@pytest.mark.parametrize("iterations", [1, 70])
+def test_descent_leaves_a_list_in_the_layout_of_the_context(hand, iterations):
+    spec = workloads.fit_mixture(n_replicas=1, n=3000, seed=8)[0]
+
+    def go(prepare):
+        with Engine(spec) as eng:
+            prepare(eng)
+            eng.minimize(iterations, 0.002, 100.0)
+            staged = eng.list_staged()
+            after_descent = _lists(eng)
+            eng.eval()
+            return staged, after_descent, _lists(eng), eng.state()
+
+    def by_hand(eng):
+        assert eng.list_staged()
+        if hand == "schedule":
+            eng.set_tuning(2, False, 4, True)
+        elif hand == "staged":
+            eng.set_list_staged(True)
+
+    a, b = go(by_hand), go(lambda eng: eng.set_list_staged(False))
+    assert a[0] is (hand != "") and b[0] is False
+    for x, y in ((a[1], b[1]), (a[2], b[2])):
+        assert np.array_equal(x[0], y[0])
+        assert all(np.array_equal(p, q) for p, q in zip(x[1], y[1]))
+    for key in ("positions", "forces", "images"):
+        assert np.array_equal(a[3][key], b[3][key]), key
