@@ -152,6 +152,7 @@ bool Engine::use_whole_steps() const {
 bool Engine::adopt_layout() {
   if (tuning_fixed_ || tuned_) return whole_steps_;
   if (v_.list_by_q != 0 && !layout_fixed_) {
+    clear_graphs();  // captured steps hold the kernels of the layout left here
     v_.list_by_q = 0;
     launch_.v = v_;
     if (initialized_) relayout_list();
@@ -943,6 +944,7 @@ cudaGraphExec_t Engine::graph_for(uint32_t steps, bool obs_last) {
 }
 
 void Engine::launch_counts(uint32_t& per_step, uint32_t& per_chain) {
+  adopt_layout();  // the layout the steps will run on
   // The cached one-step graph settles whether this driver takes conditional
   // nodes (graph_for falls back to recording the chain in every step).
   if (use_graphs_) graph_for(1, false);

@@ -44,3 +44,21 @@ def test_descent_leaves_a_list_in_the_layout_of_the_context(hand, iterations):
         assert all(np.array_equal(p, q) for p, q in zip(x[1], y[1]))
     for key in ("positions", "forces", "images"):
         assert np.array_equal(a[3][key], b[3][key]), key
+
+
+def test_steps_captured_before_the_first_evaluation_are_not_replayed_on_another_layout():
+    # more slots than whole steps in one kernel take: steps are captured graphs
+    spec = workloads.lj_lattice(n_side=53)
+
+    def go(counts_first):
+        with Engine(spec) as eng:
+            assert eng.list_staged()
+            if counts_first:
+                eng.launch_counts()
+                assert not eng.list_staged()
+            eng.profile("step", 3)
+            return eng.state()
+
+    a, b = go(True), go(False)
+    for key in ("positions", "velocities", "forces", "images"):
+        assert np.array_equal(a[key], b[key]), key
