@@ -172,6 +172,7 @@ EXPORTED = (
     "beads_debug_cells",
     "beads_debug_neighbors",
     "beads_debug_plan",
+    "beads_debug_stall",
 )
 
 _lib = None
@@ -229,6 +230,7 @@ def load():
                                          ctypes.POINTER(ctypes.c_uint32), vp]
     L.beads_debug_cells.argtypes = [vp, ctypes.c_uint32, vp]
     L.beads_debug_neighbors.argtypes = [vp, ctypes.c_uint32, ctypes.c_uint32, vp, vp]
+    L.beads_debug_stall.argtypes = [vp, ctypes.c_uint32]
     L.beads_debug_plan.argtypes = [vp, ctypes.c_uint32, ctypes.POINTER(ctypes.c_int32), vp]
     for name in EXPORTED:
         if name != "beads_ctx_destroy":

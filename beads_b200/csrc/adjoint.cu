@@ -774,6 +774,7 @@ void Engine::adjoint_restore(uint32_t c) {
 
 void Engine::adjoint_forward(uint64_t steps, uint64_t record_from, uint32_t every, double* obs) {
   TraceRange trace("beads.adjoint_forward");
+  require_whole();
   if (steps == 0) throw InvalidArgument("adjoint runs need at least one step.");
   if (record_from > steps) throw InvalidArgument("record_from must not exceed steps.");
   for (const auto& h : rep_) {
@@ -915,6 +916,7 @@ void Engine::adjoint_forward(uint64_t steps, uint64_t record_from, uint32_t ever
 void Engine::adjoint_backward(const double* obs_grad, double* grad_eps, double* grad_sigma,
                               float* grad_pos, float* grad_vel) {
   TraceRange trace("beads.adjoint_backward");
+  require_whole();
   if (!adj_ || !adj_->forward_done) throw InvalidArgument("adjoint_backward needs a forward run.");
   AdjointStore& A = *adj_;
   const uint32_t R = A.replicas;
@@ -1037,6 +1039,8 @@ void Engine::adjoint_backward(const double* obs_grad, double* grad_eps, double* 
           launch_run(launch_, run_, static_cast<uint32_t>(std::min(kReplayChunk, b - a - k)), false,
                      adjoint_run_record(static_cast<uint32_t>(k)));
         }
+        // The next restore overwrites the states, a stall's mark included.
+        wait_whole();
       } else if (use_graphs_) {
         cuda_check(cudaGraphLaunch(replay_graph_for(static_cast<uint32_t>(b - a)), stream_),
                    "replay launch");

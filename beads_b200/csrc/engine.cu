@@ -765,6 +765,7 @@ void Engine::upload_static(uint32_t n, const beads_system_desc* systems,
   run_.any_dense = launch_.any_dense;
   run_.any_sparse = launch_.any_sparse;
   run_.need_kinetic = launch_.need_kinetic;
+  run_.wait_limit = 1u << 23;
   {
     // One wave of 128-thread blocks (16 per SM) for the chain's per-slot
     // kernels when they walk the block list.
@@ -794,6 +795,8 @@ void Engine::d2h(void* dst, const void* src, size_t bytes, const char* what) {
 
 void Engine::check_status() {
   d2h(h_state_, v_.rs, rep_.size() * sizeof(ReplicaState), "status download");
+  if (h_state_[0].status & kStatusStalled) stalled_ = true;  // the first replica carries it
+  require_whole();
   for (uint32_t r = 0; r < rep_.size(); ++r) {
     const unsigned s = h_state_[r].status;
     if (s & kStatusNeighborOverflow) {
@@ -808,10 +811,6 @@ void Engine::check_status() {
       if (rep_.size() > 1) m << " (replica " << r << ")";
       throw NeighborOverflow(m.str());
     }
-    if (s & kStatusStalled) {
-      cudaMemsetAsync(run_.ctl, 0, sizeof(RunControl), stream_);
-      throw CudaError("the step kernel's blocks did not meet at a barrier.");
-    }
     if (s & kStatusFixedOverflow) {
       throw OverflowError("energy, virial or kinetic energy of a particle is not finite or "
                           "exceeds the fixed-point accumulator range (|value| < 4e18).");
@@ -821,6 +820,25 @@ void Engine::check_status() {
                       std::to_string(r) + ").");
     }
   }
+}
+
+void Engine::require_whole() {
+  if (stalled_) {
+    throw CudaError("the step kernel's blocks did not meet at a barrier; this context takes no "
+                    "further step or evaluation.");
+  }
+}
+
+void Engine::wait_whole() {
+  d2h(&h_state_[0].status, &v_.rs->status, sizeof(unsigned), "status download");
+  if (h_state_[0].status & kStatusStalled) stalled_ = true;
+  require_whole();
+}
+
+void Engine::debug_stall(uint32_t wait_limit) {
+  run_.wait_limit = wait_limit;
+  cuda_check(cudaMemsetAsync(&run_.ctl->arrive, 0xff, sizeof(uint32_t), stream_), "memset");
+  sync();
 }
 
 // Queues the download of the observables (into pinned memory): whoever waits
@@ -833,6 +851,7 @@ void Engine::queue_observables() {
 
 void Engine::eval() {
   TraceRange trace("beads.eval");
+  require_whole();
   if (adopt_layout()) {
     launch_eval(launch_, run_);
   } else {
@@ -944,6 +963,7 @@ cudaGraphExec_t Engine::graph_for(uint32_t steps, bool obs_last) {
 }
 
 void Engine::launch_counts(uint32_t& per_step, uint32_t& per_chain) {
+  require_whole();
   adopt_layout();  // the layout the steps will run on
   // The cached one-step graph settles whether this driver takes conditional
   // nodes (graph_for falls back to recording the chain in every step).
@@ -992,6 +1012,7 @@ void Engine::launch_chunk(uint32_t steps, bool obs_last) {
 bool Engine::run(uint64_t steps, uint64_t obs_every, const std::function<bool()>* poll,
                  uint64_t poll_every) {
   TraceRange trace("beads.run");
+  require_whole();
   if (!initialized_) eval();
   if (!tuned_ && !tuning_fixed_ && steps > 0) autotune();
   if (steps > 0) obs_downloaded_ = false;
@@ -1072,6 +1093,7 @@ bool Engine::run(uint64_t steps, uint64_t obs_every, const std::function<bool()>
 
 void Engine::minimize(uint32_t iterations, float dmax, float fref) {
   TraceRange trace("beads.minimize");
+  require_whole();
   StepLaunch l = launch_;
   l.sd_dmax = dmax;
   l.sd_fref = fref;
@@ -1089,7 +1111,7 @@ void Engine::minimize(uint32_t iterations, float dmax, float fref) {
       for (uint32_t it = 0; it < iterations; it += kDescentChunk) {
         launch_descent(l, run_, std::min(kDescentChunk, iterations - it));
       }
-      sync();
+      wait_whole();
     } catch (...) {
       v_.list_by_q = by_q;
       launch_.v = v_;
@@ -1131,6 +1153,7 @@ void Engine::flush_lambda() {
 }
 
 double Engine::profile(int stage, uint32_t reps) {
+  require_whole();
   if (!initialized_) eval();
   if (reps == 0) reps = 1;
   cudaEvent_t start = nullptr, stop = nullptr;
@@ -1369,6 +1392,7 @@ void Engine::debug_cells(uint32_t r, uint32_t* cell_by_tag) {
 }
 
 void Engine::set_list_staged(bool staged) {
+  require_whole();
   const bool want = staged && stage_cap_ > 0;
   layout_fixed_ = true;
   if ((v_.list_by_q != 0) == want) return;
@@ -1417,6 +1441,7 @@ void Engine::relayout_list() {
 }
 
 void Engine::debug_neighbors(uint32_t r, uint32_t cap, uint32_t* counts, uint32_t* partners) {
+  require_whole();
   if (v_.list_by_q) {
     debug_neighbors_staged(r, cap, counts, partners);
     return;

@@ -131,6 +131,13 @@ class Engine {
   // nothing is executed.
   void launch_counts(uint32_t& per_step, uint32_t& per_chain);
   void check_status();
+  // Throws once a barrier of the step kernel has run out: its blocks left their
+  // step half way, so the context takes no further step or evaluation.
+  void require_whole();
+  void wait_whole();  // waits for the stream, then the same
+  // The next step kernel's first barrier finds one arrival too few and gives up
+  // after `wait_limit` reads (test of the bounded wait).
+  void debug_stall(uint32_t wait_limit);
   // Kernel schedule of the step: threads per particle of the pair-force
   // kernel (1, 2 or 4), its batch depth (4 or 8 list entries in flight per
   // thread), whether its list loads bypass L1, and whether the second
@@ -232,6 +239,7 @@ class Engine {
   bool tuned_ = false;                 // autotune() has run
   bool whole_steps_ = false;           // steps run in k_run (run_kernel.cu), not kernel by kernel
   RunView run_{};                      // its work arrays
+  bool stalled_ = false;               // a barrier of it has run out (require_whole)
   cudaStream_t side_stream_ = nullptr;
   std::map<std::pair<uint32_t, bool>, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs_;
   std::map<uint32_t, std::pair<cudaGraph_t, cudaGraphExec_t>> replay_graphs_;

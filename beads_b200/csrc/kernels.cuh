@@ -76,6 +76,7 @@ struct RunView {
   uint32_t* chunk_sum;   // [run_scan_chunks] cell-count totals
   long long* ke_odd;     // kinetic-energy buckets of odd steps (even ones: DeviceView::ke_part)
   int any_dense, any_sparse, need_kinetic;
+  uint32_t wait_limit;   // reads of the arrival count before a barrier gives up
 };
 // What a launch of k_run records of its steps (every pointer may be null).
 // Step s of the launch (0-based) writes record k0 + s + 1: positions and

@@ -27,10 +27,11 @@ namespace {
 
 // One barrier over all blocks of the launch; `target` counts the arrivals of
 // this launch.  The wait is bounded: when the other blocks do not arrive
-// within some seconds it marks *status and returns false, and the caller
-// leaves the kernel.
-__device__ __forceinline__ bool grid_barrier(RunControl* ctl, unsigned* status,
+// within rv.wait_limit reads (some seconds) it marks *status and returns false,
+// and the caller leaves the kernel.
+__device__ __forceinline__ bool grid_barrier(const RunView& rv, unsigned* status,
                                              uint32_t& target) {
+  RunControl* ctl = rv.ctl;
   __shared__ bool ok;
   target += gridDim.x;
   __syncthreads();
@@ -41,7 +42,7 @@ __device__ __forceinline__ bool grid_barrier(RunControl* ctl, unsigned* status,
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;"
                  : "=r"(seen) : "l"(&ctl->arrive) : "memory");
     bool done = static_cast<int32_t>(seen + 1u - target) >= 0;
-    for (uint32_t tries = 0; !done && tries < (1u << 23); ++tries) {
+    for (uint32_t tries = 0; !done && tries < rv.wait_limit; ++tries) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&ctl->arrive) : "memory");
       done = static_cast<int32_t>(seen - target) >= 0;
     }
@@ -137,7 +138,7 @@ __device__ __forceinline__ bool run_scan(const DeviceView& v, const RunView& rv,
     block_exclusive_scan<kBlock>(s, total);
     if (threadIdx.x == 0) rv.chunk_sum[ch] = total;
   }
-  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  if (!grid_barrier(rv, &v.rs->status, target)) return false;
   for (uint32_t ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
     uint32_t before = 0;
     for (uint32_t k = threadIdx.x; k < ch; k += kBlock) before += rv.chunk_sum[k];
@@ -171,7 +172,7 @@ __device__ __forceinline__ bool run_scan(const DeviceView& v, const RunView& rv,
       run += cnt[k];
     }
   }
-  return grid_barrier(rv.ctl, &v.rs->status, target);
+  return grid_barrier(rv, &v.rs->status, target);
 }
 
 // The work lists of the replicas that rebuild in this step (the last block):
@@ -242,7 +243,7 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
     const ReplicaState* st = &v.rs[r];
     if (needs_rebuild<kPre>(v.rp[r], st, st->step + step + 1ull)) bin_slots(v, v.rp[r], b);
   }
-  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  if (!grid_barrier(rv, &v.rs->status, target)) return false;
   const uint32_t items = v.work_start[v.n_replicas];
   const bool reorder = rv.ctl->reorder != 0u;
   const bool wide = rv.ctl->wide != 0u;
@@ -256,7 +257,7 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
       decide_replica<kPre>(v.rp[r], st, st->step + step + 1ull);
     }
   }
-  if (items == 0u) return grid_barrier(rv.ctl, &v.rs->status, target);  // launch-uniform
+  if (items == 0u) return grid_barrier(rv, &v.rs->status, target);  // launch-uniform
   if (!wide) {
     // Cell starts, a block per rebuilding replica.
     for (uint32_t r = blockIdx.x; r < v.n_replicas; r += gridDim.x) {
@@ -290,12 +291,12 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
       }
       if (threadIdx.x == 0) start[n_cells] = run;
     }
-    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+    if (!grid_barrier(rv, &v.rs->status, target)) return false;
   } else if (!run_scan(v, rv, items, target)) {
     return false;
   }
   for (uint32_t b = b0; b < b1; ++b) scatter_block(v, b);
-  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  if (!grid_barrier(rv, &v.rs->status, target)) return false;
   if (rv.any_sparse) {
     for (uint32_t w = blockIdx.x * kBlock + threadIdx.x; w < items; w += gridDim.x * kBlock) {
       sort_cell_sparse(v, w);
@@ -306,15 +307,15 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
     sort_cell(v, v.rp[r], w - v.work_start[r], lane, sh.sort_keys[warp]);
     __syncwarp();
   }
-  if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+  if (!grid_barrier(rv, &v.rs->status, target)) return false;
   if (reorder) {
     for (uint32_t b = b0; b < b1; ++b) reorder_gather_block(v, b);
-    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+    if (!grid_barrier(rv, &v.rs->status, target)) return false;
     for (uint32_t b = b0; b < b1; ++b) reorder_commit_block(v, b);
-    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+    if (!grid_barrier(rv, &v.rs->status, target)) return false;
     if (v.excl_cap > 0u) {
       for (uint32_t b = b0; b < b1; ++b) project_exclusions_block(v, b, false);
-      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+      if (!grid_barrier(rv, &v.rs->status, target)) return false;
     }
   }
   // A thread per particle only where sparse cells alone fill the GPU several
@@ -349,7 +350,7 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
                               sh.build[warp], k - w * parts, parts);
     }
   }
-  return grid_barrier(rv.ctl, &v.rs->status, target);
+  return grid_barrier(rv, &v.rs->status, target);
 }
 
 // kPre: velocity Verlet (drift, rebuild, forces and second half-kick per step)
@@ -372,7 +373,7 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
   const bool kinetic = kEval || (kVerlet && (kObs || rv.need_kinetic != 0));
   const bool bonded = v.has_bonded != 0;
   // A launch queued behind one whose barrier ran out finds the counts in
-  // disorder (the host rearms them when it reports the error).
+  // disorder (the host takes no further call on such a context).
   if (__ldcg(&v.rs->status) & kStatusStalled) return;
   uint32_t target = 0, cur = 0xffffffffu;
   // Consecutive slot blocks and pair-force items per block: an item's
@@ -410,7 +411,7 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
     if (bonded) {
       const uint32_t terms = v.n_bond_terms + v.n_angle_terms + v.n_dihedral_terms;
       for (uint32_t t = gthread; t < terms; t += gridDim.x * kBlock) bonded_term<kObs>(v, t);
-      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return false;
+      if (!grid_barrier(rv, &v.rs->status, target)) return false;
       for (uint32_t b = b0; b < b1; ++b) {
         enter(replica_of(b));
         bonded_block<kObs>(v, p, cur, b, kVerlet, kinetic, ke, vel);
@@ -461,14 +462,14 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
     }
     if (!run_rebuild<kPre>(v, rv, rec, sh, b0, b1, 0u, 0u, target)) return;
     if (!forces(nullptr, nullptr)) return;
-    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+    if (!grid_barrier(rv, &v.rs->status, target)) return;
   }
   for (uint32_t s = 0; !kEval && s < n_steps; ++s) {
     long long* ke = (s & 1u) ? rv.ke_odd : v.ke_part;
     long long* ke_other = (s & 1u) ? v.ke_part : rv.ke_odd;
     if (!kVerlet) {
       if (!forces(nullptr, nullptr)) return;
-      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+      if (!grid_barrier(rv, &v.rs->status, target)) return;
     }
     const size_t record = (size_t)(rec.k0 + s + 1u) * v.n_slots;
     if (kVerlet && s > 0u && (kObs || rec.lam)) epilogue(s - 1u, ke_other);
@@ -497,7 +498,7 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
                       kVerlet && rec.pos ? rec.pos + record : nullptr);
       if (kVerlet && p.skin == 0.0f && threadIdx.x == 0) rv.ctl->any[s & 1u] = 1u;
     }
-    if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+    if (!grid_barrier(rv, &v.rs->status, target)) return;
     if (__ldcg(&rv.ctl->any[s & 1u]) != 0u) {  // launch-uniform
       if (!run_rebuild<kPre>(v, rv, rec, sh, b0, b1, since, s, target)) return;
       since = s + 1u;
@@ -517,7 +518,7 @@ k_run(DeviceView v, RunView rv, RunRecord rec, uint32_t n_steps, float sd_dmax, 
         }
       }
       if (!forces(ke, rec.vel ? rec.vel + record : nullptr)) return;
-      if (!grid_barrier(rv.ctl, &v.rs->status, target)) return;
+      if (!grid_barrier(rv, &v.rs->status, target)) return;
     }
   }
   if (kVerlet || kEval) {

@@ -425,3 +425,8 @@ class Engine:
         nc = np.zeros(3, np.uint32)
         _lib.check(self._lib.beads_debug_plan(self._h, replica, ctypes.byref(path), nc.ctypes.data))
         return {"path": ("direct", "regular_cell", "small_dimension")[path.value], "nc": nc}
+
+    def debug_stall(self, wait_limit: int) -> None:
+        """The next step kernel's first barrier finds one arrival too few and
+        gives up after `wait_limit` reads (beads_debug_stall)."""
+        _lib.check(self._lib.beads_debug_stall(self._h, int(wait_limit)))

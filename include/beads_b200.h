@@ -293,7 +293,7 @@ BEADS_API int beads_get_tuning(beads_ctx* ctx, int32_t* schedule);
  * and entries by slot, positions gathered from global memory.  The choice
  * never changes a result; switching rebuilds the list before the next force
  * evaluation.  A context without a call, and without a schedule fixed by hand,
- * takes the slot layout at its first evaluation (the faster one at every size);
+ * takes the slot layout at its first evaluation or descent;
  * after a call it keeps the layout set here.
  * beads_get_list_layout reports 0 when no replica can stage.
  * No reference counterpart (the reference keeps one slot-major list,
@@ -408,6 +408,13 @@ BEADS_API int beads_debug_neighbors(beads_ctx* ctx, uint32_t replica, uint32_t c
  * 2 small_dimension (neighbor_plan.cpp:107-128) and its cell grid. */
 BEADS_API int beads_debug_plan(beads_ctx* ctx, uint32_t replica, int32_t* path,
                      uint32_t* ncells3);
+/* Lets the next step kernel's blocks miss one another: its first barrier finds
+ * one arrival too few, gives up after wait_limit reads of the count, and the
+ * kernel leaves.  That call and every later step, evaluation or descent of the
+ * context then fail with BEADS_ERR_CUDA (its state was left half way through a
+ * step).  Test of the bounded wait; contexts that do not step in one kernel are
+ * not affected. */
+BEADS_API int beads_debug_stall(beads_ctx* ctx, uint32_t wait_limit);
 
 #ifdef __cplusplus
 }
