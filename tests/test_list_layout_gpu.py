@@ -62,3 +62,24 @@ def test_steps_captured_before_the_first_evaluation_are_not_replayed_on_another_
     a, b = go(True), go(False)
     for key in ("positions", "velocities", "forces", "images"):
         assert np.array_equal(a[key], b[key]), key
+
+
+def test_staged_contexts_of_different_stage_sizes_run_side_by_side():
+    # ~53 and 27 beads per cell: stages above 48 KB, of two sizes
+    specs = [workloads.lj_lattice(n_side=15, cutoff=c, check_every=1) for c in (3.6, 2.5)]
+
+    def forces(staged):
+        engines = [Engine(s) for s in specs]
+        for eng in engines:
+            eng.set_list_staged(staged)
+            eng.eval()
+        engines[0].run(3)
+        out = [eng.state() for eng in engines]
+        assert all(eng.list_staged() is staged for eng in engines)
+        for eng in engines:
+            eng.close()
+        return out
+
+    for a, b in zip(forces(True), forces(False)):
+        for key in ("positions", "forces"):
+            assert np.array_equal(a[key], b[key]), key
