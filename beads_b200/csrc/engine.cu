@@ -422,6 +422,35 @@ void Engine::upload_static(uint32_t n, const beads_system_desc* systems,
       any_dense_ |= !sparse;
     }
   }
+  // Warps that share a cell in k_build.  A warp takes its cell's particles one
+  // by one (~100 us for 20), so shares pay where the cells of a rebuild leave
+  // warps idle (4,144 are resident), or where a few crowded cells, of boxes four
+  // to ten cells wide, hold the others up; elsewhere every share reads its
+  // cell's candidates again.  Measured with 1 / 2 / 3 shares:
+  //   a rebuild, us: 729 cells of 27 beads 100 / 74 / 70, 1,000 of 20 70 / 61 / 60,
+  //     1,728 81 / 76 / 84, 3,375 95 / 100 / 103, 6,859 156 / 161 / 171,
+  //     15,625 255 / 276 / 306, 50,653 697 / 785 / 891;
+  //   a batch's step, us: 128 boxes of 256 to 32,768 beads (39,172 cells)
+  //     438 / 367 / 354, 512 of 256 to 16,384 (87,670 cells) 816 / 747 / 744,
+  //     512 of 256 to 32,768 (165,000) 1242 / - / 1257, 256 of 1,000
+  //     320 / 223 / 197, 16 of 256 to 250,000 251 / 231 / 232; without crowded
+  //     cells: 16 of 16,000 134 / 130 / 132, 64 of 8,000 219 / 214 / 219, 8 of
+  //     60,000 (2,980 cells each) 181 / 178 / 187, 4 of 250,000 324 / 330 / 352.
+  {
+    constexpr double kCrowdedOccupancy = 25.0;
+    uint64_t dense_cells = 0, crowded = 0, largest = 0;
+    for (uint32_t r = 0; r < n; ++r) {
+      const ReplicaHost& h = rep_[r];
+      if (rp[r].sparse) continue;
+      dense_cells += h.plan.n_cells;
+      largest = std::max<uint64_t>(largest, h.plan.n_cells);
+      crowded += h.n_atoms > kCrowdedOccupancy * h.plan.n_cells ? 1u : 0u;
+    }
+    // crowded cells: where at least one box per 16,384 cells has them
+    launch_.build_parts = dense_cells <= 98304u && crowded * 16384u >= dense_cells ? 3u
+                          : dense_cells <= 32768u && largest <= 2048u             ? 2u
+                                                                                  : 1u;
+  }
   n_tags_ = tags;
   total_bond_types_ = static_cast<uint32_t>(bond_types);
   total_angle_types_ = static_cast<uint32_t>(angle_types);

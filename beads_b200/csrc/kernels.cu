@@ -750,15 +750,7 @@ void launch_rebuild(const StepLaunch& l, bool force_all, bool count_build) {
     k_project_exclusions<<<l.v.n_blocks, kBlock, 0, l.stream>>>(l.v, 0);
     check_launch("project_exclusions");
   }
-  // Shares of a cell per warp.  A warp takes ~100 us for a cell of 20
-  // particles, so cells that do not fill several waves of warps (4,144) leave
-  // the last wave nearly empty: in a batch only the rebuilding replicas' cells
-  // count, a fraction of the grid.  Measured with 1 / 2 / 3 / 4 shares: 128
-  // replicas (832,000 beads) 491 / 412 / 400 / 402 us a step, 100,003 beads
-  // 46.9 / 46.6 / 47.1 / 47.2, 1,048,576 beads 238 / 240 / 245 / 250; 512
-  // replicas (3.3 M beads, some waves of rebuilding cells) 1242 / - / 1257.
-  const uint32_t parts = l.v.n_replicas > 1u ? (l.v.total_cells < 65536u ? 3u : 1u)
-                         : l.v.total_cells < 16384u ? 2u : 1u;
+  const uint32_t parts = l.build_parts;
   const uint32_t bg = (l.v.total_cells * parts + kBuildWarps - 1) / kBuildWarps;
 #define BB_BUILD(excl, q)                                                                  \
   do {                                                                                     \

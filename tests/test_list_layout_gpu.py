@@ -83,3 +83,19 @@ def test_staged_contexts_of_different_stage_sizes_run_side_by_side():
     for a, b in zip(forces(True), forces(False)):
         for key in ("positions", "forces"):
             assert np.array_equal(a[key], b[key]), key
+
+
+@pytest.mark.parametrize("n_side", [15, 16, 40])
+def test_lists_of_cells_shared_by_several_warps(n_side):
+    # cells of 27 beads, 216 cells of 19, 3,375 cells: three, two and one warp a cell
+    spec = workloads.lj_lattice(n_side=n_side, max_neighbors=128)
+    out = []
+    for by_hand in (True, False):
+        with Engine(spec) as eng:
+            if by_hand:  # the list build as a kernel of its own
+                eng.set_list_staged(False)
+                eng.set_tuning(2, False, 4, True)
+            eng.eval()
+            out.append(eng.debug_neighbors())
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
