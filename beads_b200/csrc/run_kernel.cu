@@ -298,14 +298,29 @@ __device__ __forceinline__ bool run_rebuild(const DeviceView& v, const RunView& 
   for (uint32_t b = b0; b < b1; ++b) scatter_block(v, b);
   if (!grid_barrier(rv, &v.rs->status, target)) return false;
   if (rv.any_sparse) {
-    for (uint32_t w = blockIdx.x * kBlock + threadIdx.x; w < items; w += gridDim.x * kBlock) {
-      sort_cell_sparse(v, w);
+    // A thread per cell; the few cells too big for one are taken by its whole
+    // warp at once.  (A warp walking every cell of 2,000 beads in 1.2 million
+    // cells found nothing to do for most of a step.)
+    for (uint32_t w0 = (blockIdx.x * kBuildWarps + warp) * 32u; w0 < items;
+         w0 += gridDim.x * kBlock) {
+      const uint32_t w = w0 + lane;
+      const bool left = w < items && !sort_cell_sparse(v, w) && v.rp[work_replica(v, w)].sparse;
+      uint32_t todo = __ballot_sync(kFull, left);
+      for (; todo != 0u; todo &= todo - 1u) {  // warp-uniform
+        const uint32_t wb = w0 + (uint32_t)__ffs(todo) - 1u;
+        const uint32_t r = work_replica(v, wb);
+        sort_cell(v, v.rp[r], wb - v.work_start[r], lane, sh.sort_keys[warp]);
+        __syncwarp();
+      }
     }
   }
-  for (uint32_t w = blockIdx.x * kBuildWarps + warp; w < items; w += gridDim.x * kBuildWarps) {
-    const uint32_t r = work_replica(v, w);
-    sort_cell(v, v.rp[r], w - v.work_start[r], lane, sh.sort_keys[warp]);
-    __syncwarp();
+  if (rv.any_dense) {
+    for (uint32_t w = blockIdx.x * kBuildWarps + warp; w < items; w += gridDim.x * kBuildWarps) {
+      const uint32_t r = work_replica(v, w);
+      if (v.rp[r].sparse) continue;  // warp-uniform
+      sort_cell(v, v.rp[r], w - v.work_start[r], lane, sh.sort_keys[warp]);
+      __syncwarp();
+    }
   }
   if (!grid_barrier(rv, &v.rs->status, target)) return false;
   if (reorder) {

@@ -1,0 +1,69 @@
+"""Corners of the step kernel against the same work launched kernel by kernel."""
+
+from __future__ import annotations
+
+import dataclasses
+
+import numpy as np
+import pytest
+
+from beads_b200 import workloads
+from beads_b200.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+STATE = ("positions", "velocities", "forces", "images")
+
+
+def _spec(pos, box, seed=1, **kw):
+    n = len(pos)
+    fields = dict(
+        positions=np.asarray(pos, np.float32), types=np.ones(n, np.int32),
+        velocities=np.random.default_rng(seed).standard_normal((n, 3)).astype(np.float32),
+        masses=np.ones(n, np.float32), box_bound=np.array([np.zeros(3), np.full(3, box)], np.float32),
+        rebuild_check_every=1, sort_every_rebuild=2)
+    return dataclasses.replace(workloads.lj_lattice(), **(fields | kw))
+
+
+def _droplet(side, spacing, box, gas, seed=3, **kw):
+    """A dense lattice in one corner of a box that is empty but for a gas:
+    few beads per cell on average, many in the cells of the droplet."""
+    rng = np.random.default_rng(seed)
+    drop = (np.indices((side,) * 3).reshape(3, -1).T + 0.5) * spacing
+    g = int(np.ceil(gas ** (1 / 3)))
+    sites = (np.indices((g,) * 3).reshape(3, -1).T + 0.5) * (box / g)
+    sites = sites[(sites > side * spacing + 2.0).any(1)][:gas]
+    pos = np.concatenate([drop, sites]) + rng.uniform(-0.03, 0.03, (side ** 3 + len(sites), 3))
+    return _spec(pos, box, **kw)
+
+
+def _compare(specs, calls):
+    def go(whole):
+        with Engine(specs) as eng:
+            if not whole:
+                eng.set_list_staged(False)
+                eng.set_tuning(2, False, 4, True)
+            rows = [eng.run(steps, every) for steps, every in calls]
+            return rows, [eng.state(r) for r in range(len(specs))]
+
+    a, b = go(True), go(False)
+    assert a[0] == b[0]
+    for r in range(len(specs)):
+        for key in STATE:
+            assert np.array_equal(a[1][r][key], b[1][r][key]), (r, key)
+
+
+SPARSE = {
+    # cells of about 22, of about 40, and of more than 256 beads
+    "droplet": lambda: [_droplet(8, 1.0, 48.0, 300)],
+    "tight_droplet": lambda: [_droplet(9, 0.82, 48.0, 300, sigma=np.array([[0.8]]))],
+    "crowd": lambda: [_droplet(9, 0.4, 60.0, 300, sigma=np.array([[0.38]]), dt=0.001,
+                               max_neighbors=1024)],
+    "droplet_among_dense": lambda: [_droplet(8, 1.0, 48.0, 300, seed=5)]
+    + workloads.replica_batch(2, n_min=300, n_max=900, seed=6),
+}
+
+
+@pytest.mark.parametrize("which", list(SPARSE))
+def test_crowded_cells_of_sparse_boxes(which):
+    _compare(SPARSE[which](), [(20, 10), (15, 0)])
