@@ -177,6 +177,7 @@ void Engine::autotune() {
   if (!initialized_) eval();
   if (adopt_layout()) return;
   constexpr int kWarm = 1, kReps = 4;
+  constexpr uint32_t kSeparateKickSlots = 204800;
   const bool log = [] {
     const char* e = std::getenv("BEADS_TUNE_LOG");
     return e && std::string(e) == "1";
@@ -191,7 +192,7 @@ void Engine::autotune() {
   cuda_check(cudaEventCreate(&b), "event create");
   float best = 0.f;
   StepLaunch chosen = launch_;
-  auto trial = [&](const StepLaunch& l) {
+  auto trial = [&](const StepLaunch& l, float margin = 0.0f) {
     for (int k = 0; k < kWarm; ++k) launch_forces(l, false, false, true);
     cuda_check(cudaEventRecord(a, stream_), "event record");
     for (int k = 0; k < kReps; ++k) launch_forces(l, false, false, true);
@@ -203,34 +204,44 @@ void Engine::autotune() {
       std::fprintf(stderr, "beads autotune: tpa %d depth %d no_l1 %d fuse_post %d: %.4f ms\n",
                    l.lj_tpa, l.lj_unroll, l.lj_no_l1, l.fuse_post, ms / kReps);
     }
-    if (best == 0.f || ms < best) {
+    if (best == 0.f || ms < (1.0f - margin) * best) {
       best = ms;
       chosen = l;
     }
   };
   // One coordinate at a time, each from the best so far: threads per
-  // particle {1, 2, 4} at batch depth 4 with list loads bypassing L1, then
+  // particle {2, 1, 4} at batch depth 4 with list loads bypassing L1, then
   // depth 8, then list loads through L1, then the second half-kick fused into
   // the force kernel: six trials instead of the full grid of thirteen, which
   // a short run pays for.
+  // On slot rows without bonded terms, one or four threads and depth 8 have to
+  // win by more than 8%: launched back to back, without the drift that steps have
+  // in between, they come out up to 7% ahead and still lose in the steps (us a
+  // step with 1 / 2 / 4 threads, and 2 at depth 8: LJ 105,000 beads 60 / 56 / 57,
+  // 58, 200,000 86 / 81 / 84, 84, 300,000 113 / 110 / 117, 117; four types 105,000
+  // 58 / 55 / 58, 58, 200,000 84 / 79 / 85, 84).  So does the fused kick above some
+  // 200,000 slots (fused / separate: LJ 131,000 62 / 62, 300,000 111 / 110,
+  // 1,000,000 303 / 288, 4 x 250,000 320 / 307, 128 uneven boxes 376 / 365, the
+  // 1,048,576-bead mixture 238 / 217).  Melts are near ties in the steps as well.
+  const float margin = v_.list_by_q == 0 && v_.has_bonded == 0 ? 0.08f : 0.0f;
   try {
-    for (int tpa : {1, 2, 4}) {
+    for (int tpa : {2, 1, 4}) {
       StepLaunch l = launch_;
       l.lj_tpa = tpa;
       l.lj_unroll = 4;
       l.lj_no_l1 = 1;
       l.fuse_post = 0;
-      trial(l);
+      trial(l, margin);
     }
     StepLaunch deeper = chosen;
     deeper.lj_unroll = 8;
-    trial(deeper);
+    trial(deeper, margin);
     StepLaunch l1 = chosen;
     l1.lj_no_l1 = 0;
     trial(l1);
     StepLaunch fused = chosen;
     fused.fuse_post = 1;
-    trial(fused);
+    trial(fused, v_.n_slots > kSeparateKickSlots ? margin : 0.0f);
   } catch (...) {
     cudaEventDestroy(a);
     cudaEventDestroy(b);
