@@ -136,13 +136,24 @@ void Engine::tuning(int* tpa, int* fuse_post, int* unroll, int* no_l1, int* auto
 // Steps in one persistent kernel or kernel by kernel.  k_run saves the
 // launches and the conditional node (~20 us of a step) and pays with one wave
 // of blocks sized by the list build's registers, which costs throughput once
-// the pair forces fill the GPU.  Measured, us per step, kernel by kernel ->
-// k_run: 250 beads 28 -> 13, 4,096 24 -> 14, 20,011 34 -> 25, 100,003 47 -> 46,
-// a 200,000-bead melt 140 -> 154, 1,048,576 beads 238 -> 331.
-constexpr uint32_t kWholeStepSlots = 131072;
+// the pair forces fill the GPU: from about three of its work items per block
+// on (100,000 slots).  Measured, us per step, kernel by kernel -> k_run: LJ
+// 250 beads 28 -> 13, 4,096 24 -> 13, 20,011 28 -> 20, 65,000 40 -> 38, 82,000
+// 48 -> 47, 100,003 57 -> 55, 115,000 58 -> 63, 131,000 62 -> 64; melts 30,500
+// 36 -> 29, 60,000 40 -> 37, 80,000 44 -> 42, 100,000 47 -> 47, 110,000 53 -> 58,
+// 120,000 49 -> 51; the mixture at 100,003 beads 42.4 -> 41.8, at 1,048,576
+// 238 -> 331.  A batch rebuilds some of its boxes on most steps, so it keeps the
+// gain further: 8 x 16,000 beads 84 -> 84, 16 x 8,000 88 -> 85, 128 x 1,000 (131,072
+// slots) 187 -> 130, 512 x 250 110 -> 103.
+constexpr uint32_t kWholeStepSlots = 102400;
+constexpr uint32_t kWholeBatchSlots = 131072;
+// Descents: 13 launches an iteration against none (us: 30,011 beads 51 -> 17,
+// 120,000 84 -> 43).
+constexpr uint32_t kDescentSlots = 131072;
 
 bool Engine::use_whole_steps() const {
-  return use_graphs_ && v_.n_slots <= kWholeStepSlots && !(layout_fixed_ && v_.list_by_q != 0);
+  return use_graphs_ && v_.n_slots <= (v_.n_replicas > 1u ? kWholeBatchSlots : kWholeStepSlots) &&
+         !(layout_fixed_ && v_.list_by_q != 0);
 }
 
 // Before lists are built: a context that nobody gave a layout or a schedule
@@ -1137,7 +1148,7 @@ void Engine::minimize(uint32_t iterations, float dmax, float fref) {
   StepLaunch l = launch_;
   l.sd_dmax = dmax;
   l.sd_fref = fref;
-  if (use_graphs_ && v_.n_slots <= kWholeStepSlots) {
+  if (use_graphs_ && v_.n_slots <= kDescentSlots) {
     // In k_run, on slot rows.  A context with a staged layout asked for by hand
     // leaves it for the descent; the list that is left is then laid out again,
     // so that list and layout agree between calls.

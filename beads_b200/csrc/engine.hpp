@@ -142,7 +142,7 @@ class Engine {
   // kernel (1, 2 or 4), its batch depth (4 or 8 list entries in flight per
   // thread), whether its list loads bypass L1, and whether the second
   // half-kick runs inside the last force kernel.  Every choice gives bit-identical results.  tpa = 0 hands
-  // the choice back to the engine: contexts of up to 131,072 slots then step
+  // the choice back to the engine: small contexts (use_whole_steps) then step
   // in k_run, for larger ones the autotuner times the candidates on this batch
   // at the first run (velocities and step state restored) and keeps the
   // fastest.

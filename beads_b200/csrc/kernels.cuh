@@ -69,6 +69,7 @@ struct RunControl {
   uint32_t left;     // blocks that have left it
   uint32_t any[2];   // by step parity: some slot has moved half the skin
   uint32_t reorder;  // some rebuilding replica reorders its slots
+  uint32_t next;     // shares of cells given out to the list build's warps
   uint32_t wide;     // some rebuilding replica has more cells than a block scans
 };
 struct RunView {

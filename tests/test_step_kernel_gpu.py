@@ -67,3 +67,19 @@ SPARSE = {
 @pytest.mark.parametrize("which", list(SPARSE))
 def test_crowded_cells_of_sparse_boxes(which):
     _compare(SPARSE[which](), [(20, 10), (15, 0)])
+
+
+def test_more_shares_of_cells_than_warps():
+    # 4,096 cells, shared by more warps than the launch has: some build several
+    _compare([workloads.lj_lattice(n_side=44, check_every=1, max_neighbors=128)],
+             [(12, 6), (9, 0)])
+
+
+def test_sizes_around_the_largest_context_that_steps_in_one_kernel():
+    # 102,400 slots: 128 of them or fewer beads below, at and above
+    sides, base = (102272, 102400, 102401), workloads.lj_lattice(n_side=47, max_neighbors=128)
+    for n in sides:
+        spec = dataclasses.replace(
+            base, positions=base.positions[:n], types=base.types[:n],
+            velocities=base.velocities[:n], masses=base.masses[:n], rebuild_check_every=1)
+        _compare([spec], [(8, 4)])
