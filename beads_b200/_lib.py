@@ -173,6 +173,7 @@ EXPORTED = (
     "beads_debug_neighbors",
     "beads_debug_plan",
     "beads_debug_stall",
+    "beads_debug_step_blocks",
 )
 
 _lib = None
@@ -231,6 +232,7 @@ def load():
     L.beads_debug_cells.argtypes = [vp, ctypes.c_uint32, vp]
     L.beads_debug_neighbors.argtypes = [vp, ctypes.c_uint32, ctypes.c_uint32, vp, vp]
     L.beads_debug_stall.argtypes = [vp, ctypes.c_uint32]
+    L.beads_debug_step_blocks.argtypes = [vp, ctypes.c_uint32]
     L.beads_debug_plan.argtypes = [vp, ctypes.c_uint32, ctypes.POINTER(ctypes.c_int32), vp]
     for name in EXPORTED:
         if name != "beads_ctx_destroy":

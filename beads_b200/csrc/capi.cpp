@@ -503,6 +503,13 @@ int beads_debug_plan(beads_ctx* ctx, uint32_t replica, int32_t* path, uint32_t* 
   });
 }
 
+int beads_debug_step_blocks(beads_ctx* ctx, uint32_t blocks) {
+  return guarded([&] {
+    require(ctx && ctx->engine, "NULL context.");
+    ctx->engine->debug_step_blocks(blocks);
+  });
+}
+
 int beads_debug_stall(beads_ctx* ctx, uint32_t wait_limit) {
   return guarded([&] {
     require(ctx && ctx->engine, "NULL context.");

@@ -138,6 +138,7 @@ class Engine {
   // The next step kernel's first barrier finds one arrival too few and gives up
   // after `wait_limit` reads (test of the bounded wait).
   void debug_stall(uint32_t wait_limit);
+  void debug_step_blocks(uint32_t blocks) { run_.max_blocks = blocks; }
   // Kernel schedule of the step: threads per particle of the pair-force
   // kernel (1, 2 or 4), its batch depth (4 or 8 list entries in flight per
   // thread), whether its list loads bypass L1, and whether the second

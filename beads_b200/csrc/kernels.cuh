@@ -78,6 +78,7 @@ struct RunView {
   uint32_t* chunk_sum;   // [run_scan_chunks] cell-count totals
   long long* ke_odd;     // kinetic-energy buckets of odd steps (even ones: DeviceView::ke_part)
   int any_dense, any_sparse, need_kinetic;
+  uint32_t max_blocks;   // blocks of a launch (0: one wave); lowered where the device takes fewer
   uint32_t wait_limit;   // reads of the arrival count before a barrier gives up
 };
 // What a launch of k_run records of its steps (every pointer may be null).
@@ -99,12 +100,12 @@ constexpr int kRunBlocksPerSm = 7;  // resident blocks: the list build's registe
 // n_steps velocity-Verlet steps or descent iterations of every replica;
 // slot-layout lists only.  observables: energies and virial of every step
 // (DeviceView::obs keeps the last step's).
-void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables,
+void launch_run(const StepLaunch& l, RunView& rv, uint32_t n_steps, bool observables,
                 const RunRecord& rec = RunRecord{});
-void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps);
+void launch_descent(const StepLaunch& l, RunView& rv, uint32_t n_steps);
 // The evaluation of the current state: pending Berendsen scales applied, every
 // list built, forces, energies, virial and kinetic energy.
-void launch_eval(const StepLaunch& l, const RunView& rv);
+void launch_eval(const StepLaunch& l, RunView& rv);
 uint32_t run_scan_chunks(uint32_t total_cells);
 
 }  // namespace bb

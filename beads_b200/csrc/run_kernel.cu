@@ -19,8 +19,11 @@
 #include "step_device.cuh"
 
 #include <algorithm>
+#include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <utility>
 
 namespace bb {
 namespace {
@@ -589,24 +592,33 @@ void check(cudaError_t e) {
   }
 }
 
+// Blocks of one wave of `kernel` on the current device (kept per kernel and
+// device).
+uint32_t wave_of(const void* kernel) {
+  static std::mutex mutex;
+  static std::map<std::pair<int, const void*>, uint32_t> waves;
+  int device = 0, sms = 0, per_sm = 0;
+  check(cudaGetDevice(&device));
+  const std::lock_guard<std::mutex> lock(mutex);
+  uint32_t& wave = waves[{device, kernel}];
+  if (wave == 0u) {
+    check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, 0));
+    wave = (uint32_t)(sms * per_sm);
+  }
+  return wave;
+}
+
 template <int kPre, bool kObs, int kNt, bool kSmall>
-void launch_as(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uint32_t n_steps) {
+void launch_as(const StepLaunch& l, RunView& rv, const RunRecord& rec, uint32_t n_steps) {
   auto* kernel = k_run<kPre, kObs, kNt, kSmall>;
   // One wave at most.  Pair-force items of a small system leave blocks idle,
   // but a rebuild shares its cells over every warp, and barriers take the same
   // time up to about two blocks per SM.
-  static const uint32_t wave = [&] {
-    int device = 0, sms = 0, per_sm = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) {
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, 0);
-    }
-    check(e);
-    return (uint32_t)(sms * per_sm);
-  }();
+  const uint32_t most =
+      rv.max_blocks != 0u ? rv.max_blocks : wave_of(reinterpret_cast<const void*>(kernel));
+  uint32_t blocks = std::min(most, std::max(kMinGrid, l.v.n_blocks * (uint32_t)kRunTpa));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(std::min(wave, std::max(kMinGrid, l.v.n_blocks * (uint32_t)kRunTpa)));
   cfg.blockDim = dim3(kBlock);
   cfg.stream = l.stream;
   cudaLaunchAttribute attr[1];
@@ -614,11 +626,25 @@ void launch_as(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uin
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  check(cudaLaunchKernelEx(&cfg, kernel, l.v, rv, rec, n_steps, l.sd_dmax, l.sd_fref));
+  // A process that has part of the SMs may be refused a wave of all of them: any
+  // number of blocks takes the same steps, so half as many are tried, and kept
+  // for the context.
+  for (;;) {
+    cfg.gridDim = dim3(blocks);
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, kernel, l.v, rv, rec, n_steps, l.sd_dmax, l.sd_fref);
+    if (e != cudaErrorCooperativeLaunchTooLarge || blocks <= 1u) {
+      check(e);
+      return;
+    }
+    (void)cudaGetLastError();
+    blocks = (blocks + 1u) / 2u;
+    rv.max_blocks = blocks;
+  }
 }
 
 template <int kPre, bool kObs, int kNt>
-void launch_one(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uint32_t n_steps) {
+void launch_one(const StepLaunch& l, RunView& rv, const RunRecord& rec, uint32_t n_steps) {
   if (l.v.n_blocks * (uint32_t)kRunTpa <= kSmallItems) {
     launch_as<kPre, kObs, kNt, true>(l, rv, rec, n_steps);
   } else {
@@ -629,7 +655,7 @@ void launch_one(const StepLaunch& l, const RunView& rv, const RunRecord& rec, ui
 // The LJ table specialisation of the batch: its coefficients in registers for
 // one or two types.
 template <int kPre, bool kObs>
-void launch_types(const StepLaunch& l, const RunView& rv, const RunRecord& rec, uint32_t n_steps) {
+void launch_types(const StepLaunch& l, RunView& rv, const RunRecord& rec, uint32_t n_steps) {
   switch (l.lj_types) {
     case 1: launch_one<kPre, kObs, 1>(l, rv, rec, n_steps); break;
     case 2: launch_one<kPre, kObs, 2>(l, rv, rec, n_steps); break;
@@ -639,7 +665,7 @@ void launch_types(const StepLaunch& l, const RunView& rv, const RunRecord& rec, 
 
 }  // namespace
 
-void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool observables,
+void launch_run(const StepLaunch& l, RunView& rv, uint32_t n_steps, bool observables,
                 const RunRecord& rec) {
   if (observables) {
     launch_types<kPreVerlet, true>(l, rv, rec, n_steps);
@@ -648,11 +674,11 @@ void launch_run(const StepLaunch& l, const RunView& rv, uint32_t n_steps, bool o
   }
 }
 
-void launch_descent(const StepLaunch& l, const RunView& rv, uint32_t n_steps) {
+void launch_descent(const StepLaunch& l, RunView& rv, uint32_t n_steps) {
   launch_types<kPreDescent, false>(l, rv, RunRecord{}, n_steps);
 }
 
-void launch_eval(const StepLaunch& l, const RunView& rv) {
+void launch_eval(const StepLaunch& l, RunView& rv) {
   launch_one<kPreEval, true, 0>(l, rv, RunRecord{}, 1);
 }
 

@@ -430,3 +430,8 @@ class Engine:
         """The next step kernel's first barrier finds one arrival too few and
         gives up after `wait_limit` reads (beads_debug_stall)."""
         _lib.check(self._lib.beads_debug_stall(self._h, int(wait_limit)))
+
+    def debug_step_blocks(self, blocks: int) -> None:
+        """Largest number of blocks of the context's step kernels
+        (beads_debug_step_blocks); 0 for as many as are resident at once."""
+        _lib.check(self._lib.beads_debug_step_blocks(self._h, int(blocks)))

@@ -408,6 +408,10 @@ BEADS_API int beads_debug_neighbors(beads_ctx* ctx, uint32_t replica, uint32_t c
  * 2 small_dimension (neighbor_plan.cpp:107-128) and its cell grid. */
 BEADS_API int beads_debug_plan(beads_ctx* ctx, uint32_t replica, int32_t* path,
                      uint32_t* ncells3);
+/* Largest number of blocks of the context's step kernels (0: as many as are
+ * resident at once).  A number the device refuses is halved until it is taken,
+ * as for a process that has part of the SMs.  Any number takes the same steps. */
+BEADS_API int beads_debug_step_blocks(beads_ctx* ctx, uint32_t blocks);
 /* Lets the next step kernel's blocks miss one another: its first barrier finds
  * one arrival too few, gives up after wait_limit reads of the count, and the
  * kernel leaves.  That call and every later step, evaluation or descent of the

@@ -83,3 +83,27 @@ def test_sizes_around_the_largest_context_that_steps_in_one_kernel():
             base, positions=base.positions[:n], types=base.types[:n],
             velocities=base.velocities[:n], masses=base.masses[:n], rebuild_check_every=1)
         _compare([spec], [(8, 4)])
+
+
+@pytest.mark.parametrize("blocks", [1, 3, 100, 60000])
+def test_any_number_of_blocks_takes_the_same_steps(blocks):
+    """60,000 blocks are more than a GPU holds at once: the launch is refused
+    and made with fewer.  The large system has work for that many."""
+    large = blocks > 1000
+    specs = ([workloads.lj_lattice(n_side=45, check_every=1, max_neighbors=128)] if large else
+             [_droplet(8, 1.0, 48.0, 200), workloads.polymer_melt(n_chains=8, beads=40, seed=4,
+                                                                  max_neighbors=96)])
+
+    def go(limit):
+        with Engine(specs) as eng:
+            if limit:
+                eng.debug_step_blocks(limit)
+            eng.minimize(3, 0.002, 100.0)
+            rows = [eng.eval(), eng.run(12, 6)]
+            return rows, [eng.state(r) for r in range(len(specs))]
+
+    a, b = go(blocks), go(0)
+    assert a[0] == b[0]
+    for x, y in zip(a[1], b[1]):
+        for key in STATE:
+            assert np.array_equal(x[key], y[key]), key
