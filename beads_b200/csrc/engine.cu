@@ -1015,7 +1015,11 @@ cudaGraphExec_t Engine::graph_for(uint32_t steps, bool obs_last) {
 
 void Engine::launch_counts(uint32_t& per_step, uint32_t& per_chain) {
   require_whole();
-  adopt_layout();  // the layout the steps will run on
+  if (adopt_layout()) {  // (also settles the layout the steps will run on)
+    per_step = 1;
+    per_chain = 0;
+    return;
+  }
   // The cached one-step graph settles whether this driver takes conditional
   // nodes (graph_for falls back to recording the chain in every step).
   if (use_graphs_) graph_for(1, false);

@@ -127,8 +127,8 @@ class Engine {
   // Kernels one MD step launches under the current schedule, and the
   // kernels of one rebuild chain when that chain runs only on rebuild steps
   // (0 when every step launches it: no conditional graph node).  Counted
-  // as the kernel nodes of one captured step, also where steps run in k_run;
-  // nothing is executed.
+  // as the kernel nodes of one captured step; nothing is executed.  1 and 0
+  // where steps run in k_run, up to 16 of them per launch.
   void launch_counts(uint32_t& per_step, uint32_t& per_chain);
   void check_status();
   // Throws once a barrier of the step kernel has run out: its blocks left their

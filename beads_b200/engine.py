@@ -392,7 +392,8 @@ class Engine:
     def launch_counts(self) -> dict:
         """Kernels per MD step and per rebuild chain under the current
         schedule (see beads_launch_counts); per_rebuild_chain is 0 when every
-        step launches the chain."""
+        step launches the chain, and per_step 1 as well where up to 16 steps
+        of a call share one launch."""
         per_step = ctypes.c_uint32()
         per_chain = ctypes.c_uint32()
         _lib.check(self._lib.beads_launch_counts(self._h, ctypes.byref(per_step),

@@ -354,11 +354,11 @@ BEADS_API int beads_counters(beads_ctx* ctx, uint32_t replica, uint64_t* counter
  * (counters[3] of beads_counters counts those runs).  *per_rebuild_chain is 0
  * when every step launches the chain itself (no conditional graph node, or
  * graphs switched off with BEADS_GRAPHS=0); *per_step then includes it.
- * Counted as the kernel nodes of one captured step; nothing runs.  A context of
- * up to 131,072 particle slots whose schedule nobody fixed does not step that
- * way: it takes up to 16 steps, rebuilds included, per launch of one kernel,
- * and the counts are those of the steps it would capture.  No counterpart in
- * the reference (measurement). */
+ * Counted as the kernel nodes of one captured step; nothing runs.  1 and 0 for a
+ * context that takes its steps, rebuilds included, in one kernel, up to 16 of a
+ * call per launch (single systems of up to 102,400 particle slots and batches of
+ * up to 131,072 whose schedule nobody fixed).  No counterpart in the reference
+ * (measurement). */
 BEADS_API int beads_launch_counts(beads_ctx* ctx, uint32_t* per_step,
                                   uint32_t* per_rebuild_chain);
 

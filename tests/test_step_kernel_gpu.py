@@ -107,3 +107,12 @@ def test_any_number_of_blocks_takes_the_same_steps(blocks):
     for x, y in zip(a[1], b[1]):
         for key in STATE:
             assert np.array_equal(x[key], y[key]), key
+
+
+def test_launch_counts_of_a_context_that_steps_in_one_kernel():
+    with Engine(workloads.lj_lattice(n_side=8)) as eng:
+        assert eng.launch_counts() == {"per_step": 1, "per_rebuild_chain": 0}
+        eng.run(5)
+        assert eng.launch_counts() == {"per_step": 1, "per_rebuild_chain": 0}
+        eng.set_tuning(2, True, 4, True)  # kernel by kernel
+        assert eng.launch_counts()["per_step"] == 4
