@@ -18,8 +18,8 @@
 // at once; a block never straddles two replicas; the rebuild decision is taken
 // on the device so a captured step loop needs no host round trip; totals are
 // reduced in 64-bit fixed point so they do not depend on block scheduling;
-// bonded forces are gathered per particle (each thread evaluates the terms its
-// particle belongs to) so no force atomics exist anywhere.
+// bonded terms are evaluated once each and their members' forces gathered per
+// particle, so no force atomics exist anywhere.
 #include "kernels.cuh"
 #include "device_util.cuh"
 #include "step_device.cuh"

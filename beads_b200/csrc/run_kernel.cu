@@ -1,6 +1,6 @@
 // run_kernel.cu -- whole MD steps in one persistent kernel.
 //
-// A step launched kernel by kernel costs about 28 us before any work: five
+// A step launched kernel by kernel costs about 20 us before any work: five
 // kernels at ~0.6 us each inside a captured graph, their own latencies, and
 // the conditional node that holds the rebuild chain (8 us when it is not
 // taken, 17 us when it is, on top of its kernels).  k_run takes a stretch of
