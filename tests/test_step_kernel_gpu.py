@@ -30,9 +30,9 @@ def _droplet(side, spacing, box, gas, seed=3, **kw):
     few beads per cell on average, many in the cells of the droplet."""
     rng = np.random.default_rng(seed)
     drop = (np.indices((side,) * 3).reshape(3, -1).T + 0.5) * spacing
-    g = int(np.ceil(gas ** (1 / 3)))
+    g = max(1, int(np.ceil(gas ** (1 / 3))))
     sites = (np.indices((g,) * 3).reshape(3, -1).T + 0.5) * (box / g)
-    sites = sites[(sites > side * spacing + 2.0).any(1)][:gas]
+    sites = sites[(sites > side * spacing + 2.0).any(1)][:gas].reshape(-1, 3)
     pos = np.concatenate([drop, sites]) + rng.uniform(-0.03, 0.03, (side ** 3 + len(sites), 3))
     return _spec(pos, box, **kw)
 
@@ -116,3 +116,38 @@ def test_launch_counts_of_a_context_that_steps_in_one_kernel():
         assert eng.launch_counts() == {"per_step": 1, "per_rebuild_chain": 0}
         eng.set_tuning(2, True, 4, True)  # kernel by kernel
         assert eng.launch_counts()["per_step"] == 4
+
+
+DESCENTS = {
+    "fluid": lambda: [_droplet(9, 1.0, 9.6, 0, sort_every_rebuild=3)],
+    "no_skin": lambda: [_droplet(7, 1.0, 7.6, 0, cutoff_buffer=0.0, cutoff=2.4)],
+    # exclusions, bonded terms, a thermostat, boxes of several sizes and types
+    "batch": lambda: [workloads.polymer_melt(n_chains=8, beads=40, seed=4, max_neighbors=128),
+                      _droplet(8, 1.0, 48.0, 150, seed=2)]
+    + workloads.fit_mixture(n_replicas=2, n=700, seed=3),
+}
+
+
+@pytest.mark.parametrize("which", list(DESCENTS))
+@pytest.mark.parametrize("iterations", [1, 63, 64, 65, 129])
+def test_descent_gives_the_bits_of_separate_launches(which, iterations, monkeypatch):
+    """BEADS_GRAPHS=0 launches every kernel of an iteration by itself."""
+    specs = DESCENTS[which]()
+
+    def go(cuts):
+        with Engine(specs) as eng:
+            for n in cuts:
+                eng.minimize(n, 0.004, 50.0)
+            states = [eng.state(r) for r in range(len(specs))]
+            eng.eval()
+            return states, [eng.state(r)["forces"] for r in range(len(specs))]
+
+    cuts = [[iterations], [40, iterations - 40] if iterations > 40 else [iterations]]
+    whole = [go(c) for c in cuts]
+    monkeypatch.setenv("BEADS_GRAPHS", "0")
+    apart = [go(c) for c in cuts]
+    for a, b in zip(whole, apart):
+        for r in range(len(specs)):
+            for key in ("positions", "images"):
+                assert np.array_equal(a[0][r][key], b[0][r][key]), (r, key)
+            assert np.array_equal(a[1][r], b[1][r]), r
