@@ -1039,8 +1039,10 @@ void Engine::adjoint_backward(const double* obs_grad, double* grad_eps, double* 
           launch_run(launch_, run_, static_cast<uint32_t>(std::min(kReplayChunk, b - a - k)), false,
                      adjoint_run_record(static_cast<uint32_t>(k)));
         }
-        // The next restore overwrites the states, a stall's mark included.
-        wait_whole();
+        // The next restore overwrites the states, a stall's mark included: it is
+        // read with the wait below.
+        cuda_check(cudaMemcpyAsync(&h_state_[0].status, &v_.rs->status, sizeof(unsigned),
+                                   cudaMemcpyDeviceToHost, stream_), "status copy");
       } else if (use_graphs_) {
         cuda_check(cudaGraphLaunch(replay_graph_for(static_cast<uint32_t>(b - a)), stream_),
                    "replay launch");
@@ -1055,6 +1057,10 @@ void Engine::adjoint_backward(const double* obs_grad, double* grad_eps, double* 
       }
     }
     sync();
+    if (whole_steps_ && !A.store_all) {
+      if (h_state_[0].status & kStatusStalled) stalled_ = true;
+      require_whole();
+    }
     flags.resize(static_cast<size_t>(b - a + 1) * R);
     d2h(flags.data(), A.seg_flags, flags.size() * sizeof(uint32_t), "flags");
     // The list each forward step m used: built at the replica's last rebuild
