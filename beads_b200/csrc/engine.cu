@@ -449,8 +449,8 @@ void Engine::upload_static(uint32_t n, const beads_system_desc* systems,
   // warps idle (4,144 are resident), or where a few crowded cells, of boxes four
   // to ten cells wide, hold the others up; elsewhere every share reads its
   // cell's candidates again.  Measured with 1 / 2 / 3 shares:
-  //   a rebuild, us: 729 cells of 27 beads 100 / 74 / 70, 1,000 of 20 70 / 61 / 60,
-  //     1,728 81 / 76 / 84, 3,375 95 / 100 / 103, 6,859 156 / 161 / 171,
+  //   a rebuild, us: 216 cells of 23 beads 64 / 53 / 49, 729 of 27 100 / 74 / 70,
+  //     1,000 of 20 70 / 61 / 60, 1,728 81 / 76 / 84, 3,375 95 / 100 / 103, 6,859 156 / 161 / 171,
   //     15,625 255 / 276 / 306, 50,653 697 / 785 / 891;
   //   a batch's step, us: 128 boxes of 256 to 32,768 beads (39,172 cells)
   //     438 / 367 / 354, 512 of 256 to 16,384 (87,670 cells) 816 / 747 / 744,
@@ -469,9 +469,10 @@ void Engine::upload_static(uint32_t n, const beads_system_desc* systems,
       crowded += h.n_atoms > kCrowdedOccupancy * h.plan.n_cells ? 1u : 0u;
     }
     // crowded cells: where at least one box per 16,384 cells has them
-    launch_.build_parts = dense_cells <= 98304u && crowded * 16384u >= dense_cells ? 3u
-                          : dense_cells <= 32768u && largest <= 2048u             ? 2u
-                                                                                  : 1u;
+    const bool three = dense_cells <= 1024u ||
+                       (dense_cells <= 98304u && crowded * 16384u >= dense_cells);
+    const bool two = dense_cells <= 32768u && largest <= 2048u;
+    launch_.build_parts = three ? 3u : two ? 2u : 1u;
   }
   n_tags_ = tags;
   total_bond_types_ = static_cast<uint32_t>(bond_types);

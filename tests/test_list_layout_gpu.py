@@ -85,9 +85,10 @@ def test_staged_contexts_of_different_stage_sizes_run_side_by_side():
             assert np.array_equal(a[key], b[key]), key
 
 
-@pytest.mark.parametrize("n_side", [15, 16, 40])
+@pytest.mark.parametrize("n_side", [15, 16, 30, 40])
 def test_lists_of_cells_shared_by_several_warps(n_side):
-    # cells of 27 beads, 216 cells of 19, 3,375 cells: three, two and one warp a cell
+    # cells of 27 beads, 216 cells of 19, 1,331 cells, 3,375 cells: three, three,
+    # two and one warp a cell
     spec = workloads.lj_lattice(n_side=n_side, max_neighbors=128)
     out = []
     for by_hand in (True, False):
