@@ -233,7 +233,8 @@ void Engine::autotune() {
   // 58 / 55 / 58, 58, 200,000 84 / 79 / 85, 84).  So does the fused kick above some
   // 200,000 slots (fused / separate: LJ 131,000 62 / 62, 300,000 111 / 110,
   // 1,000,000 303 / 288, 4 x 250,000 320 / 307, 128 uneven boxes 376 / 365, the
-  // 1,048,576-bead mixture 238 / 217).  Melts are near ties in the steps as well.
+  // 1,048,576-bead mixture 238 / 217).  Loads through L1 have to win by 2%: they are
+  // within 0.5% either way.  Melts are near ties in the steps as well.
   const float margin = v_.list_by_q == 0 && v_.has_bonded == 0 ? 0.08f : 0.0f;
   try {
     for (int tpa : {2, 1, 4}) {
@@ -249,7 +250,7 @@ void Engine::autotune() {
     trial(deeper, margin);
     StepLaunch l1 = chosen;
     l1.lj_no_l1 = 0;
-    trial(l1);
+    trial(l1, margin * 0.25f);
     StepLaunch fused = chosen;
     fused.fuse_post = 1;
     trial(fused, v_.n_slots > kSeparateKickSlots ? margin : 0.0f);
