@@ -296,7 +296,9 @@ class Engine:
         """Pair forces from shared-memory cell tiles (True) or global gathers
         (False); the same bits either way (beads_set_list_layout).  Once set,
         this layout is kept; a context without a call (and without a schedule
-        fixed by hand) takes the slot layout at its first evaluation."""
+        fixed by hand) takes the slot layout at its first evaluation or descent.
+        The staged layout's kernel keeps four list entries in flight whatever
+        batch_depth says."""
         _lib.check(self._lib.beads_set_list_layout(self._h, 1 if staged else 0))
 
     def list_staged(self) -> bool:
