@@ -108,7 +108,8 @@ class Engine {
   // Pair forces from shared-memory cell tiles (list rows by cell order, stage
   // indices as entries) or from global gathers (rows by slot, slot entries).
   // Contexts start staged when some replica qualifies and leave that layout at
-  // their first evaluation unless it was asked for (adopt_layout); switching
+  // their first evaluation or descent unless it was asked for (adopt_layout);
+  // switching
   // rebuilds the list before the next force evaluation.  Results are the same
   // bits.
   void set_list_staged(bool staged);
