@@ -228,16 +228,19 @@ void Engine::autotune() {
   // the force kernel: six trials instead of the full grid of thirteen, which
   // a short run pays for.
   // On slot rows without bonded terms, one or four threads and depth 8 have to
-  // win by more than 8%: launched back to back, without the drift that steps have
-  // in between, they come out up to 7% ahead and still lose in the steps (us a
-  // step with 1 / 2 / 4 threads, and 2 at depth 8: LJ 105,000 beads 60 / 56 / 57,
-  // 58, 200,000 86 / 81 / 84, 84, 300,000 113 / 110 / 117, 117; four types 105,000
-  // 58 / 55 / 58, 58, 200,000 84 / 79 / 85, 84).  So does the fused kick above some
-  // 200,000 slots (fused / separate: LJ 131,000 62 / 62, 300,000 111 / 110,
-  // 1,000,000 303 / 288, 4 x 250,000 320 / 307, 128 uneven boxes 376 / 365, the
-  // 1,048,576-bead mixture 238 / 217).  Loads through L1 have to win by 2%: they are
-  // within 0.5% either way.  Melts are near ties in the steps as well.
-  const float margin = v_.list_by_q == 0 && v_.has_bonded == 0 ? 0.08f : 0.0f;
+  // win by more than 15%: launched back to back, without the drift that steps
+  // have in between, they come out up to 10% ahead and lose in the steps at every
+  // size and state measured (us a step with 1 / 2 / 4 threads, and 2 at depth 8: LJ
+  // 105,000 beads 60 / 56 / 57, 58, 200,000 86 / 81 / 84, 84, 300,000 113 / 110 /
+  // 117, 117; four types 105,000 58 / 55 / 58, 58, 200,000 84 / 79 / 85, 84).  The
+  // fused kick above some 200,000 slots has to win by 8%: timed so it comes out
+  // ahead of the separate one on sorted slots too, where it loses (fused /
+  // separate: LJ 131,000 62 / 62, 300,000 111 / 110, 1,000,000 303 / 288, 4 x 250,000
+  // 320 / 307, 128 uneven boxes 376 / 365, the 1,048,576-bead mixture 238 / 217).
+  // Loads through L1 have to win by 2%: they are within 0.5% either way.  Melts are
+  // near ties in the steps as well.
+  const bool settled = v_.list_by_q == 0 && v_.has_bonded == 0;
+  const float margin = settled ? 0.15f : 0.0f;
   try {
     for (int tpa : {2, 1, 4}) {
       StepLaunch l = launch_;
@@ -252,10 +255,10 @@ void Engine::autotune() {
     trial(deeper, margin);
     StepLaunch l1 = chosen;
     l1.lj_no_l1 = 0;
-    trial(l1, margin * 0.25f);
+    trial(l1, settled ? 0.02f : 0.0f);
     StepLaunch fused = chosen;
     fused.fuse_post = 1;
-    trial(fused, v_.n_slots > kSeparateKickSlots ? margin : 0.0f);
+    trial(fused, settled && v_.n_slots > kSeparateKickSlots ? 0.08f : 0.0f);
   } catch (...) {
     cudaEventDestroy(a);
     cudaEventDestroy(b);
