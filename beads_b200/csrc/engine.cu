@@ -144,15 +144,18 @@ void Engine::tuning(int* tpa, int* fuse_post, int* unroll, int* no_l1, int* auto
 // 120,000 49 -> 51; the mixture at 100,003 beads 42.4 -> 41.8, at 1,048,576
 // 238 -> 331.  A batch rebuilds some of its boxes on most steps, so it keeps the
 // gain further: 8 x 16,000 beads 84 -> 84, 16 x 8,000 88 -> 85, 128 x 1,000 (131,072
-// slots) 187 -> 130, 512 x 250 110 -> 103.
+// slots) 187 -> 130, 512 x 250 110 -> 103.  So do fluids of more than two types,
+// whose coefficients come from shared memory either way: 104,000 beads 54 -> 52,
+// 118,000 59 -> 57, 131,000 59 -> 56.
 constexpr uint32_t kWholeStepSlots = 102400;
-constexpr uint32_t kWholeBatchSlots = 131072;
+constexpr uint32_t kWholeWideSlots = 131072;
 // Descents: 13 launches an iteration against none (us: 30,011 beads 51 -> 17,
 // 120,000 84 -> 43).
 constexpr uint32_t kDescentSlots = 131072;
 
 bool Engine::use_whole_steps() const {
-  return use_graphs_ && v_.n_slots <= (v_.n_replicas > 1u ? kWholeBatchSlots : kWholeStepSlots) &&
+  const bool wide = v_.n_replicas > 1u || (launch_.lj_types > 2 && v_.has_bonded == 0);
+  return use_graphs_ && v_.n_slots <= (wide ? kWholeWideSlots : kWholeStepSlots) &&
          !(layout_fixed_ && v_.list_by_q != 0);
 }
 

@@ -356,9 +356,9 @@ BEADS_API int beads_counters(beads_ctx* ctx, uint32_t replica, uint64_t* counter
  * graphs switched off with BEADS_GRAPHS=0); *per_step then includes it.
  * Counted as the kernel nodes of one captured step; nothing runs.  1 and 0 for a
  * context that takes its steps, rebuilds included, in one kernel, up to 16 of a
- * call per launch (single systems of up to 102,400 particle slots and batches of
- * up to 131,072 whose schedule nobody fixed).  No counterpart in the reference
- * (measurement). */
+ * call per launch (systems of up to 102,400 particle slots, batches and unbonded
+ * systems of more than two types of up to 131,072, whose schedule nobody fixed).
+ * No counterpart in the reference (measurement). */
 BEADS_API int beads_launch_counts(beads_ctx* ctx, uint32_t* per_step,
                                   uint32_t* per_rebuild_chain);
 

@@ -151,3 +151,16 @@ def test_descent_gives_the_bits_of_separate_launches(which, iterations, monkeypa
             for key in ("positions", "images"):
                 assert np.array_equal(a[0][r][key], b[0][r][key]), (r, key)
             assert np.array_equal(a[1][r], b[1][r]), r
+
+
+def test_more_than_two_types_step_in_one_kernel_up_to_131072_slots():
+    base = workloads.lj_lattice(n_side=48, max_neighbors=128, check_every=1)
+    scale = np.array([1.0, 0.9, 1.1])
+    spec = dataclasses.replace(
+        base, types=(np.arange(base.n) % 3 + 1).astype(np.int32),
+        epsilon=np.sqrt(np.outer(scale, scale)), sigma=np.full((3, 3), 1.0))
+    with Engine(spec) as eng:
+        assert eng.launch_counts()["per_step"] == 1
+    _compare([spec], [(8, 4)])
+    with Engine(base) as eng:  # one type, the same size: kernel by kernel
+        assert eng.launch_counts()["per_step"] > 1
